@@ -12,6 +12,7 @@
 #include "bicgstab.h"
 #include "gmres.h"
 #include "mixed.h"
+#include "pcg_coop.h"
 
 #include <math.h>
 #include <float.h>
@@ -19,6 +20,7 @@
 #include <stdio.h>
 #include <string.h>
 
+#include <algorithm>
 #include <string>
 #include <vector>
 
@@ -206,6 +208,9 @@ struct phgGpuSystem_ {
 
     // solver
     DevBuf<double> x, r, p, Ap, partials, hist, sums;
+    DevBuf<int32_t> coop_cols;             // their copy of the matrix
+    DevBuf<double> coop_vals;
+    DevBuf<double> coop_xch;               // exchange memory of the one-kernel solvers
     DevBuf<PcgState> st;
     DevBuf<unsigned> ticket;
     DevBuf<int64_t> tmp64;
@@ -258,6 +263,8 @@ struct phgGpuSystem_ {
     int64_t sell2_total = 0, q16_total = 0;   // stored entries (padding included)
     int64_t pair_entries = 0, q16_entries = 0; // the same, known from the slice widths
     double tune_ms[kTuneCandidates] = {};
+    bool plan_set = false;            // the plan is the caller's (phgGpuSetSpMVPlan)
+    bool plan_due = false;            // a solve on the current matrix needed no plan: chosen when asked for
 
     // mixed-precision solver
     DevBuf<float> r32, p32, Ap32, y32, D32;
@@ -680,6 +687,11 @@ SpmvPlan make_plan(phgGpuSystem *s, int kind, int param) {
     return P;
 }
 
+// Whether the caller chose the product layout for the current matrix shape.
+bool plan_forced(const phgGpuSystem *s) {
+    return s->plan_set && s->tuned && s->tuned_n == s->n && s->tuned_nnz == s->nnz;
+}
+
 // Chooses the fastest SpMV layout for the current matrix shape by timing
 // every candidate on the system's stream (once per (n, nnz)).  With
 // build_layout false a plan chosen before is kept without building its
@@ -726,6 +738,7 @@ int tune_spmv(phgGpuSystem *s, bool build_layout = true) {
     cudaEventDestroy(b);
     s->plan = make_plan(s, kTuneKind[best], kTuneParam[best]);
     s->unroll32 = 0;
+    s->plan_set = false;
     s->tuned = true;
     s->tuned_n = s->n;
     s->tuned_nnz = s->nnz;
@@ -835,6 +848,9 @@ int phgGpuDestroy(phgGpuSystem *s) {
     s->tmp64.release();
     s->st.release();
     s->ticket.release();
+    s->coop_xch.release();
+    s->coop_cols.release();
+    s->coop_vals.release();
     s->status.release();
     if (s->h_st) cudaFreeHost(s->h_st);
     if (s->h_sums) cudaFreeHost(s->h_sums);
@@ -1496,6 +1512,7 @@ int phgGpuSetSpMVPlan(phgGpuSystem *s, int kind, int param) {
                         "65536-column windows");
     }
     s->plan = make_plan(s, kind, param);
+    s->plan_set = true;
     s->tuned = true;
     s->tuned_n = s->n;
     s->tuned_nnz = s->nnz;
@@ -1523,6 +1540,11 @@ int phgGpuSetSpMVPlan32(phgGpuSystem *s, int layout, int unroll) {
 
 int phgGpuGetSpMVPlan(phgGpuSystem *s, int *kind, int *param, double *times_ms) {
     if (s == nullptr) return fail(PHG_GPU_ERR_ARG, "null system");
+    if (s->plan_due && s->assembled) {
+        CHECK_RC(set_device(s));
+        CHECK_RC(tune_spmv(s));
+        s->plan_due = false;
+    }
     if (!s->tuned) return fail(PHG_GPU_ERR_STATE, "the SpMV layout is chosen at the first solve or product");
     if (kind) *kind = s->plan.kind;
     if (param) *param = s->plan.kind == SPMV_CSR ? s->plan.lpr : s->plan.unroll;
@@ -1567,11 +1589,34 @@ int phgGpuGetLaunchCount(phgGpuSystem *s, int64_t *count) {
 
 namespace {
 
-// FP64 Jacobi-PCG on the assembled matrix with right-hand side `drhs`
-// (device), iterating on s->x (initial guess in, solution out).  Returns the
-// iteration count or a negative error code.
-int pcg_core(phgGpuSystem *s, const double *drhs, double rtol, double btol, double atol, int maxit,
-             double *dhist, double *residual) {
+// The solve as one cooperative kernel (pcg_coop.cu), state left in s->h_st.
+// Returns 1, or 0 when the kernel does not take it: a matrix whose vectors
+// exceed the SMs' shared memory, a very long row, or a product layout the
+// caller asked for (phgGpuSetSpMVPlan).
+int pcg_one_kernel(phgGpuSystem *s, const double *drhs, double rtol, double btol, double atol, int maxit,
+                   double *dhist) {
+    const int64_t n = s->n;
+    if (plan_forced(s)) return 0;
+    const int64_t entries = pcg_coop_entries(n, s->nnz);
+    if (entries < 0) return 0;
+    CHECK_RC(s->coop_cols.ensure((size_t)entries));
+    CHECK_RC(s->coop_vals.ensure((size_t)entries));
+    CHECK_RC(s->coop_xch.ensure((size_t)coop_exchange_doubles()));
+    CK(cudaMemsetAsync(s->coop_xch.p, 0, sizeof(double) * coop_exchange_doubles(), s->stream));
+    const PcgRun run{CsrView{n, s->rp.p, s->ci.p, s->va.p}, s->nnz, s->coop_cols.p, s->coop_vals.p, s->x.p, s->p.p,
+                     drhs, s->diag.p, rtol, btol, atol, maxit, dhist, s->coop_xch.p, s->st.p};
+    CK(launch_pcg_coop(run, s->stream));
+    s->launches += 1;
+    CK(cudaMemcpyAsync(s->h_st, s->st.p, sizeof(PcgState), cudaMemcpyDeviceToHost, s->stream));
+    CK(cudaStreamSynchronize(s->stream));
+    if (s->h_st->status == kStatusDeclined) return 0;
+    s->plan_due = true;
+    return 1;
+}
+
+// The solve as launches in a graph loop on the plan's layout, state left in
+// s->h_st.
+int pcg_graph(phgGpuSystem *s, const double *drhs, double rtol, double btol, double atol, int maxit, double *dhist) {
     const int64_t n = s->n;
     CK(cudaMemsetAsync(s->ticket.p, 0, sizeof(unsigned) * kRedTickets, s->stream));
     // ||b|| and |x|_1 (solver-phg.c:498-518)
@@ -1583,9 +1628,9 @@ int pcg_core(phgGpuSystem *s, const double *drhs, double rtol, double btol, doub
     auto is_zero = [](double a) { return fabs(a) < 10.0 * DBL_MIN; };   // utils.h:451
     if (is_zero(rb)) {
         CK(cudaMemsetAsync(s->x.p, 0, sizeof(double) * n, s->stream));
-        if (residual) *residual = 0.0;
         if (dhist) CK(cudaMemsetAsync(dhist, 0, sizeof(double), s->stream));
-        return 0;
+        *s->h_st = PcgState{};
+        return PHG_GPU_OK;
     }
     CsrView A{n, s->rp.p, s->ci.p, s->va.p};
     CHECK_RC(tune_spmv(s));
@@ -1652,10 +1697,25 @@ int pcg_core(phgGpuSystem *s, const double *drhs, double rtol, double btol, doub
     if (plain_limit) s->h_st->status = kStatusPassLimit;
     if (s->plain_graphs) s->launches += 3 * (int64_t)kGraphChunk * plain_passes;
     else s->launches += 3 * (int64_t)kGraphChunk * s->h_st->passes + s->h_st->passes;
+    return PHG_GPU_OK;
+}
+
+// FP64 Jacobi-PCG on the assembled matrix with right-hand side `drhs`
+// (device), iterating on s->x (initial guess in, solution out).  Returns the
+// iteration count or a negative error code.
+int pcg_core(phgGpuSystem *s, const double *drhs, double rtol, double btol, double atol, int maxit,
+             double *dhist, double *residual) {
+    int rc = pcg_one_kernel(s, drhs, rtol, btol, atol, maxit, dhist);
+    if (rc < 0) return rc;
+    if (rc == 0) {
+        rc = pcg_graph(s, drhs, rtol, btol, atol, maxit, dhist);
+        if (rc < 0) return rc;
+    }
     const int nits = s->h_st->nits;
     if (residual) *residual = s->h_st->residual;
     if (s->h_st->status == kStatusPassLimit)
-        return fail(PHG_GPU_ERR_STATE, "PCG: the iteration loop exceeded its pass bound");
+        return fail(PHG_GPU_ERR_STATE, "PCG: the iteration loop exceeded its bound");
+    if (s->h_st->status == kStatusBadStart) return fail(PHG_GPU_ERR_NAN, "PCG: zero or non-finite diagonal");
     if (s->h_st->status == PCG_BREAKDOWN)
         warn("PCG stopped after %d iterations: the matrix may not be SPD", nits);
     if (s->h_st->status == PCG_NONFINITE)

@@ -1,0 +1,30 @@
+// FP64 Jacobi-PCG as one cooperative kernel (pcg_coop.cu).
+#pragma once
+#include "solve.h"
+
+namespace phgb {
+
+// One solve of A x = b from the initial guess in x: p (n) is the direction
+// the product gathers, the other vectors stay on chip.
+struct PcgRun {
+    CsrView A;
+    int64_t nnz;
+    int32_t *cols;       // the blocks' copy of the matrix: pcg_coop_entries() each
+    double *vals;
+    double *x, *p;
+    const double *b, *D;
+    double rtol, btol, atol;
+    int maxit;
+    double *hist;        // optional: ||r|| after each iteration, [0] = ||r0||
+    double *exchange;    // coop_exchange_doubles(), zero before the launch
+    PcgState *st;        // out: nits, residual, status
+};
+
+int coop_exchange_doubles();
+
+// Entries of the matrix copy a solve of n rows and nnz entries makes on the
+// current device, -1 when it is too large for the kernel.
+int64_t pcg_coop_entries(int64_t n, int64_t nnz);
+cudaError_t launch_pcg_coop(const PcgRun &R, cudaStream_t s);
+
+}  // namespace phgb

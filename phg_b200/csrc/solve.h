@@ -38,6 +38,10 @@ struct PcgState {
 
 // Status of a solve whose graph loop ran out of passes (a safeguard).
 constexpr int kStatusPassLimit = 3;
+// Status of a solve whose initial r.z is not finite (a zero or non-finite diagonal).
+constexpr int kStatusBadStart = 4;
+// Status of a solve the one-kernel solver did not take (a row longer than it holds).
+constexpr int kStatusDeclined = 5;
 
 struct CsrView {
     int64_t n;
