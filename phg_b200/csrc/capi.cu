@@ -12,6 +12,7 @@
 #include "bicgstab.h"
 #include "gmres.h"
 #include "mixed.h"
+#include "mixed_coop.h"
 #include "pcg_coop.h"
 
 #include <math.h>
@@ -210,6 +211,9 @@ struct phgGpuSystem_ {
     DevBuf<double> x, r, p, Ap, partials, hist, sums;
     DevBuf<int32_t> coop_cols;             // their copy of the matrix
     DevBuf<double> coop_vals;
+    DevBuf<float> coop_vals32;
+    DevBuf<MixedResult> mixed_out;
+    MixedResult *h_mixed = nullptr;
     DevBuf<double> coop_xch;               // exchange memory of the one-kernel solvers
     DevBuf<PcgState> st;
     DevBuf<unsigned> ticket;
@@ -265,6 +269,7 @@ struct phgGpuSystem_ {
     double tune_ms[kTuneCandidates] = {};
     bool plan_set = false;            // the plan is the caller's (phgGpuSetSpMVPlan)
     bool plan_due = false;            // a solve on the current matrix needed no plan: chosen when asked for
+    bool plan32_set = false, plan32_due = false;   // the same for the FP32 product
 
     // mixed-precision solver
     DevBuf<float> r32, p32, Ap32, y32, D32;
@@ -648,6 +653,7 @@ int tune_spmv32(phgGpuSystem *s) {
     }
     cudaEventDestroy(a);
     cudaEventDestroy(b);
+    s->plan32_set = false;
     s->kind32 = kTune32Kind[best];
     s->unroll32 = kTune32Unroll[best];
     s->tuned32_n = s->n;
@@ -851,6 +857,9 @@ int phgGpuDestroy(phgGpuSystem *s) {
     s->coop_xch.release();
     s->coop_cols.release();
     s->coop_vals.release();
+    s->coop_vals32.release();
+    s->mixed_out.release();
+    if (s->h_mixed) cudaFreeHost(s->h_mixed);
     s->status.release();
     if (s->h_st) cudaFreeHost(s->h_st);
     if (s->h_sums) cudaFreeHost(s->h_sums);
@@ -1305,6 +1314,35 @@ int phgGpuMatVec(phgGpuSystem *s, const double *x, double *y) {
     return PHG_GPU_OK;
 }
 
+// The mixed solve as one cooperative kernel (mixed_coop.cu) on s->x, its result
+// in s->h_mixed.  Returns 1, or 0 when the kernel does not take it: a matrix
+// whose vectors exceed the SMs' shared memory, a very long row, or an FP32
+// layout the caller asked for (phgGpuSetSpMVPlan32).
+static int mixed_one_kernel(phgGpuSystem *s, double rtol, double btol, double atol, int maxit) {
+    const int64_t n = s->n;
+    if (s->plan32_set && s->unroll32 != 0 && s->tuned32_n == n && s->tuned32_nnz == s->nnz) return 0;
+    const int64_t entries = mixed_coop_entries(n, s->nnz);
+    if (entries < 0) return 0;
+    CHECK_RC(s->coop_cols.ensure((size_t)entries));
+    CHECK_RC(s->coop_vals.ensure((size_t)entries));
+    CHECK_RC(s->coop_vals32.ensure((size_t)entries));
+    CHECK_RC(s->coop_xch.ensure((size_t)coop_exchange_doubles()));
+    CHECK_RC(s->u32.ensure((size_t)n));
+    CHECK_RC(s->mixed_out.ensure(1));
+    if (s->h_mixed == nullptr) CK(cudaMallocHost((void **)&s->h_mixed, sizeof(MixedResult)));
+    CK(cudaMemsetAsync(s->coop_xch.p, 0, sizeof(double) * coop_exchange_doubles(), s->stream));
+    const MixedRun run{CsrView{n, s->rp.p, s->ci.p, s->va.p}, s->nnz, s->coop_cols.p, s->coop_vals32.p, s->coop_vals.p,
+                       s->x.p, s->u32.p, s->rhs.p, s->diag.p, rtol, btol, atol, 0.1, maxit, s->coop_xch.p,
+                       s->mixed_out.p};
+    CK(launch_mixed_coop(run, s->stream));
+    s->launches += 1;
+    CK(cudaMemcpyAsync(s->h_mixed, s->mixed_out.p, sizeof(MixedResult), cudaMemcpyDeviceToHost, s->stream));
+    CK(cudaStreamSynchronize(s->stream));
+    if (s->h_mixed->status == kStatusDeclined) return 0;
+    s->plan_due = s->plan32_due = true;
+    return 1;
+}
+
 int phgGpuSolverPCGMixed(phgGpuSystem *s, double rtol, double btol, double atol, int maxit, double *x,
                          double *residual, int *nupdates) {
     g_last_warning.clear();
@@ -1313,9 +1351,31 @@ int phgGpuSolverPCGMixed(phgGpuSystem *s, double rtol, double btol, double atol,
     if (maxit < 0) return fail(PHG_GPU_ERR_ARG, "maxit < 0");
     CHECK_RC(set_device(s));
     CHECK_RC(solver_buffers(s));
-    CHECK_RC(tune_spmv(s, false));
     const int64_t n = s->n;
     const size_t un = (size_t)n;
+    CHECK_RC(copy_in(s, s->x.p, x, un));
+    const int one = mixed_one_kernel(s, rtol, btol, atol, maxit);
+    if (one < 0) return one;
+    if (one > 0) {
+        const MixedResult &m = *s->h_mixed;
+        switch (m.status) {
+        case kStatusBadStart: return fail(PHG_GPU_ERR_NAN, "phgGpuSolverPCGMixed: zero or non-finite diagonal");
+        case PCG_NONFINITE: return fail(PHG_GPU_ERR_NAN, "mixed PCG: non-finite residual");
+        case kStatusPassLimit:
+            return fail(PHG_GPU_ERR_STATE, "mixed PCG: the iteration loop exceeded its bound");
+        case PCG_BREAKDOWN:
+            // as the FP64 PCG: warn, keep the iterate, report its FP64 residual
+            warn("mixed PCG stopped after %d iterations: the matrix may not be SPD", m.nits);
+            break;
+        default: break;
+        }
+        CHECK_RC(copy_out(s, x, s->x.p, un));
+        CK(cudaStreamSynchronize(s->stream));
+        if (residual) *residual = m.residual;
+        if (nupdates) *nupdates = m.nupdates;
+        return m.nits;
+    }
+    CHECK_RC(tune_spmv(s, false));
     CHECK_RC(s->r32.ensure(un));
     CHECK_RC(s->p32.ensure(un));
     CHECK_RC(s->Ap32.ensure(un));
@@ -1325,7 +1385,6 @@ int phgGpuSolverPCGMixed(phgGpuSystem *s, double rtol, double btol, double atol,
     CHECK_RC(s->s32.ensure(un));
     CHECK_RC(s->gst.ensure(1));
     if (s->h_gst_mixed == nullptr) CK(cudaMallocHost((void **)&s->h_gst_mixed, sizeof(GearState)));
-    CHECK_RC(copy_in(s, s->x.p, x, un));
     CK(cudaMemsetAsync(s->ticket.p, 0, sizeof(unsigned) * kRedTickets, s->stream));
     CHECK_RC(tune_spmv32(s));   // builds the chosen FP32 layout for this matrix
     if (s->plan.kind == SPMV_Q16) CHECK_RC(ensure_q16(s));   // the FP64 plan's layout (checked by tune_spmv)
@@ -1533,6 +1592,7 @@ int phgGpuSetSpMVPlan32(phgGpuSystem *s, int layout, int unroll) {
                     "65536-column windows");
     s->kind32 = layout;
     s->unroll32 = unroll;
+    s->plan32_set = true;
     s->tuned32_n = s->n;
     s->tuned32_nnz = s->nnz;
     return PHG_GPU_OK;
@@ -1544,6 +1604,8 @@ int phgGpuGetSpMVPlan(phgGpuSystem *s, int *kind, int *param, double *times_ms) 
         CHECK_RC(set_device(s));
         CHECK_RC(tune_spmv(s));
         s->plan_due = false;
+        if (s->plan32_due) CHECK_RC(tune_spmv32(s));
+        s->plan32_due = false;
     }
     if (!s->tuned) return fail(PHG_GPU_ERR_STATE, "the SpMV layout is chosen at the first solve or product");
     if (kind) *kind = s->plan.kind;

@@ -11,10 +11,10 @@
 // its loads are coalesced.  The 32 gathers of a step are the same neighbour of
 // consecutive rows and share cache lines.
 //
-// A block with fewer slices than warps splits each slice's steps into `parts`
-// ranges for as many warps, whose sums are added in order; where there are more
-// (slice, part) units than warps, the warps take them as they come free, so
-// that long slices do not queue behind one another.
+// Where slices are few or rows long, H = 2 or 4 lanes share a row (its entries
+// in turn), so that a slice is the work of H warps; where there are more such
+// units than warps, the warps take them as they come free, so that long units
+// do not queue behind one another.
 #pragma once
 #include "common.cuh"
 #include "grid_sync.cuh"
@@ -22,93 +22,82 @@
 
 namespace phgb {
 
-constexpr int kCoopMaxRowLen = 1024;   // longer rows would be a lane's serial work
-
-// Parts per slice for a matrix of n rows and nnz entries whose blocks have at
-// most that many slices: enough units for the 32 warps, and where rows are
-// long up to six units a warp, so that the longest slice (a P2 vertex row has
-// 65 entries against 25 on average, a P3 one 175 against 41) does not outlast
-// the rest; each part keeps four steps or more.  Measured per iteration, parts
-// 1 / 2 / 4: P1 36k rows (8 slices) 9.2 / 8.3 / 8.5 us, P1 133k (28) 10.8 / 11.7
-// / 14.1, P2 69k (15) 19.4 / 14.6 / 11.9, P2 250k (53) 28.1 / 24.9 / 25.2, P2
-// 531k (113) 47.6 / 47.4 / 70.8, P3 227k (48) 51.3 / 35.7 / 32.2.
-inline int coop_parts(int64_t slices, int64_t n, int64_t nnz) {
-    const int64_t units = nnz >= 16 * n ? 192 : kCoopWarps;
-    int p = 1;
-    while (p < 4 && 2 * p * slices <= units && nnz >= 8 * p * n) p *= 2;
-    return p;
-}
+constexpr int kCoopMaxRowLen = 1024;   // longer rows would be a few lanes' serial work
 
 // Shared memory of the row bookkeeping of a block with that many slices: the
-// sums of all parts but the first, each unit's first entry, and the rows'
-// lengths.
-constexpr int64_t coop_rows_bytes(int64_t slices, int parts) {
-    return slices * (32 * 8 * (parts - 1) + 4 * parts + 32 * 2);
+// rows' lengths and each unit's first entry.
+__host__ __device__ constexpr int64_t coop_rows_bytes(int64_t slices, int lanes) {
+    return slices * (4 * lanes + 32 * 2);
 }
 
+// Places of the calling block: 32 for each of its slices.
+__device__ __forceinline__ int coop_places(int64_t n) {
+    return 32 * (int)(((n + 31) / 32 - blockIdx.x + gridDim.x - 1) / gridDim.x);
+}
+
+template <int H>
 struct CoopRows {
-    int slices, parts;      // of the block; its slice k is slice blockIdx.x + gridDim.x * k
+    int slices;             // of the block; its slice k is slice blockIdx.x + gridDim.x * k
     unsigned n;             // rows of the matrix
-    double *extra;          // shared, [parts - 1][32 slices]
-    int32_t *off;           // shared, [slices][parts] first entry of each unit
+    int32_t *off;           // shared, [H slices] first entry of each unit
     uint16_t *len;          // shared, [32 slices] row lengths
     int *next;              // shared, the next unit to take
-    int32_t *cols;          // global, the matrix in step order
-    double *vals;
+    int32_t *cols;          // global, the matrix's columns in step order
 
-    // Places 0 .. places() - 1 are the block's rows, in slice order; row()
+    // Places 0 .. 32 slices - 1 are the block's rows, in slice order; row()
     // gives the matrix row, which is n or more for the last slice's padding.
-    __device__ __forceinline__ int places() const { return 32 * slices; }
     __device__ __forceinline__ unsigned row(int place) const {
         return 32u * (blockIdx.x + gridDim.x * (unsigned)(place >> 5)) + (place & 31);
     }
 
-    __device__ __forceinline__ CoopRows(int64_t rows, int slice_parts, void *shared, int *next_unit, int32_t *c,
-                                        double *v) {
-        const int64_t all = (rows + 31) / 32;
+    __device__ __forceinline__ CoopRows(int64_t rows, void *shared, int *next_unit, int32_t *c) {
         n = (unsigned)rows;
-        slices = (int)((all - blockIdx.x + gridDim.x - 1) / gridDim.x);
-        parts = slice_parts;
-        extra = (double *)shared;
-        off = (int32_t *)(extra + (parts - 1) * 32 * slices);
-        len = (uint16_t *)(off + parts * slices);
+        slices = coop_places(rows) / 32;
+        off = (int32_t *)shared;
+        len = (uint16_t *)(off + H * slices);
         next = next_unit;
         cols = c;
-        vals = v;
     }
 
-    // Steps [j0, j1) of a unit of a slice of `width` steps.
-    __device__ __forceinline__ int first_step(int part, int width) const { return (width * part) / parts; }
+    // Unit u is 32 / H consecutive places, lane `lane` at this one.
+    __device__ __forceinline__ int place_of(int unit, int lane) const { return (32 * unit + lane) / H; }
+    // Entries of a row of l the lane takes: lane % H, lane % H + H, ...
+    __device__ __forceinline__ int own(int l, int lane) const { return (l + H - 1 - lane % H) / H; }
 
-    // Copies the CSR rows of the block into step order.  All threads call it,
-    // the block's next barrier completes it.
-    __device__ __forceinline__ void build(const CsrView &A) const {
+    // Copies the CSR rows of the block into step order: columns to cols, and
+    // put(place, value) the values.  All threads call it, the block's next
+    // barrier completes it.
+    template <class Put>
+    __device__ __forceinline__ void build(const CsrView &A, Put put) const {
         constexpr int U = 4;
         const int lane = threadIdx.x & 31;
         const unsigned lt = (1u << lane) - 1u;
         if (threadIdx.x == 0) *next = kCoopWarps;
-        for (int k = threadIdx.x >> 5; k < slices; k += kCoopWarps) {
-            const unsigned r = row(32 * k + lane);
+        for (int unit = threadIdx.x >> 5; unit < H * slices; unit += kCoopWarps) {
+            const int place = place_of(unit, lane);
+            const unsigned r = row(place);
             const int32_t b = A.rp[min(r, n)], e = A.rp[min(r + 1, n)];
-            const int l = e - b, width = __reduce_max_sync(0xffffffffu, (unsigned)l);
-            int at = __shfl_sync(0xffffffffu, b, 0), part = 0;
-            len[32 * k + lane] = (uint16_t)l;
-            for (int j = 0; j < width || part < parts; j += U) {   // one more turn starts parts at the end
+            const int mine = own(e - b, lane), width = __reduce_max_sync(0xffffffffu, (unsigned)mine);
+            int at = __shfl_sync(0xffffffffu, b, 0);
+            if (lane % H == 0) len[place] = (uint16_t)(e - b);
+            if (lane == 0) off[unit] = at;
+            for (int j = 0; j < width; j += U) {
                 int32_t c[U];
                 double v[U];
 #pragma unroll
                 for (int u = 0; u < U; u++) {
-                    c[u] = j + u < l ? __ldg(&A.ci[b + j + u]) : 0;
-                    v[u] = j + u < l ? __ldg(&A.va[b + j + u]) : 0.0;
+                    const bool in = j + u < mine;
+                    const int32_t q = b + (j + u) * H + lane % H;
+                    c[u] = in ? __ldg(&A.ci[q]) : 0;
+                    v[u] = in ? __ldg(&A.va[q]) : 0.0;
                 }
 #pragma unroll
                 for (int u = 0; u < U; u++) {
-                    for (; part < parts && first_step(part, width) == j + u; part++)
-                        if (lane == 0) off[k * parts + part] = at;
-                    const unsigned m = __ballot_sync(0xffffffffu, j + u < l);
-                    if (j + u < l) {
-                        cols[at + __popc(m & lt)] = c[u];
-                        vals[at + __popc(m & lt)] = v[u];
+                    const unsigned m = __ballot_sync(0xffffffffu, j + u < mine);
+                    if (j + u < mine) {
+                        const int q = at + __popc(m & lt);
+                        cols[q] = c[u];
+                        put(q, v[u]);
                     }
                     at += __popc(m);
                 }
@@ -117,39 +106,18 @@ struct CoopRows {
     }
 
     // y[place] = (A x)_row for the block's places (shared memory, zero in the
-    // padding).  x is read with plain loads: other blocks write it between
-    // barriers.  All threads call it, with y and the parts free to write; y is
-    // complete when it returns.
-    __device__ __forceinline__ void product(const double *x, double *y) const {
-        constexpr int U = 8;
-        const int lane = threadIdx.x & 31, units = slices * parts;
-        const unsigned lt = (1u << lane) - 1u;
+    // padding), values `vals` in step order.  x is read with plain loads: other
+    // blocks write it between barriers.  All threads call it, with y free to
+    // write; y is complete when it returns.  ORDERED: each row's sum takes its
+    // entries in CSR order, one by one, whatever H (the sums of the launched
+    // SELL products); otherwise the lanes' sums are added.
+    template <bool ORDERED, class V>
+    __device__ __forceinline__ void product(const V *vals, const V *x, V *y) const {
+        const int lane = threadIdx.x & 31, units = H * slices;
         for (int unit = threadIdx.x >> 5; unit < units;) {
-            const int k = unit / parts, part = unit % parts;
-            const int l = len[32 * k + lane], width = __reduce_max_sync(0xffffffffu, (unsigned)l);
-            const int j1 = first_step(part + 1, width), le = min(l, j1);
-            int at = off[unit];
-            double acc = 0.0;
-            for (int j = first_step(part, width); j < j1; j += U) {
-                int32_t c[U];
-                double v[U];
-#pragma unroll
-                for (int u = 0; u < U; u++) {
-                    const unsigned m = __ballot_sync(0xffffffffu, j + u < le);
-                    c[u] = -1;
-                    v[u] = 0.0;
-                    if (j + u < le) {
-                        const int q = at + __popc(m & lt);
-                        c[u] = load_once(cols + q);
-                        v[u] = load_once(vals + q);
-                    }
-                    at += __popc(m);
-                }
-#pragma unroll
-                for (int u = 0; u < U; u++)
-                    if (c[u] >= 0) acc += v[u] * x[c[u]];
-            }
-            (part == 0 ? y : extra + (part - 1) * 32 * slices)[32 * k + lane] = acc;
+            const int place = place_of(unit, lane);
+            const V acc = row_sum<ORDERED>(vals, x, off[unit], len[place]);
+            if (lane % H == 0) y[place] = acc;
             unit = units;
             if (units > kCoopWarps) {
                 if (lane == 0) unit = atomicAdd(next, 1);
@@ -158,22 +126,103 @@ struct CoopRows {
         }
         __syncthreads();
         if (threadIdx.x == 0) *next = kCoopWarps;   // before the next product: every caller has a barrier between
-        if (parts > 1) {
-            for (int i = threadIdx.x; i < 32 * slices; i += kCoopThreads) {
-                double s = y[i];
-                for (int q = 0; q < parts - 1; q++) s += extra[q * 32 * slices + i];
-                y[i] = s;
-            }
-            __syncthreads();
+    }
+
+    // f(place, (A x)_row) in one lane for each of the block's places: the
+    // product (ordered) without a place to keep it, the units dealt to the
+    // warps in turn.
+    template <class V, class F>
+    __device__ __forceinline__ void product_each(const V *vals, const V *x, F f) const {
+        const int lane = threadIdx.x & 31;
+        for (int unit = threadIdx.x >> 5; unit < H * slices; unit += kCoopWarps) {
+            const int place = place_of(unit, lane);
+            const V acc = row_sum<true>(vals, x, off[unit], len[place]);
+            if (lane % H == 0) f(place, acc);
         }
     }
 
 private:
+    // Sum of the lane's row, of length l, in every lane of the row; the
+    // unit's entries start at `at`.  FP32 entries are loaded a batch ahead of
+    // the gathers they feed (FP64 ones would not fit the registers).
+    template <bool ORDERED, class V>
+    __device__ __forceinline__ V row_sum(const V *vals, const V *x, int at, int l) const {
+        constexpr int U = 8;
+        constexpr bool ahead = sizeof(V) == 4;
+        const int lane = threadIdx.x & 31, mine = own(l, lane);
+        const int width = __reduce_max_sync(0xffffffffu, (unsigned)mine);
+        const unsigned lt = (1u << lane) - 1u;
+        V acc = (V)0;
+        int32_t c[U], cn[ahead ? U : 1];
+        V v[U], vn[ahead ? U : 1];
+        auto load = [&](int j, int32_t *cc, V *vv) {
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                const unsigned m = __ballot_sync(0xffffffffu, j + u < mine);
+                cc[u] = -1;
+                vv[u] = (V)0;
+                if (j + u < mine) {
+                    const int q = at + __popc(m & lt);
+                    cc[u] = load_once(cols + q);
+                    vv[u] = load_once(vals + q);
+                }
+                at += __popc(m);
+            }
+        };
+        if (ahead) load(0, cn, vn);
+        for (int j = 0; j < width; j += U) {
+            if (ahead) {
+#pragma unroll
+                for (int u = 0; u < U; u++) {
+                    c[u] = cn[ahead ? u : 0];
+                    v[u] = vn[ahead ? u : 0];
+                }
+                load(j + U, cn, vn);
+            } else {
+                load(j, c, v);
+            }
+            V xv[U];
+#pragma unroll
+            for (int u = 0; u < U; u++) xv[u] = c[u] >= 0 ? x[c[u]] : (V)0;
+            if constexpr (ORDERED && H > 1) {
+#pragma unroll
+                for (int u = 0; u < U; u++)
+#pragma unroll
+                    for (int h = 0; h < H; h++) {
+                        const bool in = (j + u) * H + h < l;
+                        if constexpr (sizeof(V) == 4) {
+                            const V p = __shfl_sync(0xffffffffu, __fmul_rn(v[u], xv[u]), h, H);
+                            if (in) acc = __fadd_rn(acc, p);
+                        } else {
+                            const V vh = __shfl_sync(0xffffffffu, v[u], h, H), xh = __shfl_sync(0xffffffffu, xv[u], h, H);
+                            if (in) acc = fma(vh, xh, acc);
+                        }
+                    }
+            } else {
+#pragma unroll
+                for (int u = 0; u < U; u++)
+                    if (c[u] >= 0) {
+                        if constexpr (sizeof(V) == 4) acc = fma_free(acc, v[u], xv[u]);   // as the launched FP32 products
+                        else acc = fma(v[u], xv[u], acc);
+                    }
+            }
+        }
+        if constexpr (!ORDERED)
+#pragma unroll
+            for (int o = H / 2; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o, H);
+        return acc;
+    }
+
     // Matrix words are read once per product: they stay out of L1, which the
     // gathers need.
     static __device__ __forceinline__ int32_t load_once(const int32_t *p) {
         int32_t v;
         asm volatile("ld.global.L1::no_allocate.s32 %0, [%1];" : "=r"(v) : "l"(p));
+        return v;
+    }
+    static __device__ __forceinline__ float load_once(const float *p) {
+        float v;
+        asm volatile("ld.global.L1::no_allocate.f32 %0, [%1];" : "=f"(v) : "l"(p));
         return v;
     }
     static __device__ __forceinline__ double load_once(const double *p) {
@@ -182,5 +231,73 @@ private:
         return v;
     }
 };
+
+// Lanes per row (at most `most`) for a matrix of n rows and nnz entries whose
+// blocks have at most that many slices: enough units for the 32 warps, two a
+// warp where rows have 16 entries or more and six where they have 32 or more
+// (P3's vertex rows, 175 entries against 41 on average, outlast the rest
+// otherwise), while a lane keeps four entries or more.  Measured us per
+// iteration with 1 / 2 / 4 lanes: FP64 PCG P1 36k rows (8 slices) 8.7 / 7.9 /
+// 8.0, P1 133k (28) 10.4 / 10.9 / 13.2, P2 69k (15) 16.1 / 13.9 / 11.3, P2 250k
+// (53) 22.5 / 23.9 / 24.5, P2 531k (113) 38.5 / 44.6 / 47.3, P3 227k (48) 39.9 /
+// 31.5 / 30.8; mixed PCG, whose ordered sums cost more lanes more, P1 36k 7.5 /
+// 7.2 / 8.4, P2 69k 12.6 / 11.1 / 12.2, P2 250k 18.7 / 21.4 / 26.6, P3 227k 29.6 /
+// 25.6 / 30.7.
+inline int coop_lanes(int64_t slices, int64_t n, int64_t nnz, int most) {
+    const int64_t units = nnz >= 32 * n ? 192 : nnz >= 16 * n ? 64 : kCoopWarps;
+    int h = 1;
+    while (h < most && 2 * h * slices <= units && nnz >= 8 * h * n) h *= 2;
+    return h;
+}
+
+// The launch of a one-kernel solver: blocks, lanes a row and shared memory
+// (`row_bytes` of vectors a row, and the row bookkeeping); false when it is too
+// large.
+//
+// Shared memory a solve takes at most: what it takes the L1 cache loses, and
+// the product's gathers need that.  With 122 KB a block (P2, 531k rows) an
+// iteration of the FP64 PCG takes 38.5 us (58.5 as separate launches); with 208
+// KB, in an earlier form of the product, 71 against 47.5.
+constexpr int64_t kCoopMaxSmem = 136 * 1024;
+// A block per this many entries (a row's vector work counted as four) while
+// there are SMs: below that the barriers of more blocks cost what they save.
+constexpr int64_t kCoopBlockWork = 4096;
+
+struct CoopSplit {
+    int blocks = 0, lanes = 1;
+    int64_t smem = 0;
+};
+
+inline bool coop_split(int64_t n, int64_t nnz, int64_t row_bytes, int most_lanes, CoopSplit *out) {
+    int dev = 0, coop = 0, sms = 0, most = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    if (!coop) return false;
+    if (sms > kCoopMaxBlocks) sms = kCoopMaxBlocks;
+    const int64_t slices = ceil_div(n, 32);
+    int64_t G = ceil_div(nnz + 4 * n, kCoopBlockWork);
+    if (G > slices) G = slices;
+    if (G > sms) G = sms;
+    const int64_t per = ceil_div(slices, G);
+    out->blocks = (int)G;
+    out->lanes = coop_lanes(per, n, nnz, most_lanes);
+    out->smem = 32 * per * row_bytes + coop_rows_bytes(per, out->lanes);
+    return out->smem <= kCoopMaxSmem && out->smem <= most - 4096;   // 4 KB of static shared memory at most
+}
+
+// Cooperative launch of kernel(run) with that split.
+template <class Run>
+inline cudaError_t coop_launch(void (*kernel)(Run), const Run &run, const CoopSplit &sp, cudaStream_t s) {
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCoopMaxSmem);
+    if (e != cudaSuccess) return e;
+    Run r = run;
+    void *args[] = {(void *)&r};
+    return cudaLaunchCooperativeKernel((const void *)kernel, dim3(sp.blocks), dim3(kCoopThreads), args, (size_t)sp.smem, s);
+}
 
 }  // namespace phgb

@@ -13,9 +13,9 @@
 // and the latency of the phases between them; from 100,000 rows on the product,
 // which reads the matrix from L2 (up to some 10 million entries) at the rate
 // its gathers allow.  Time per iteration against the same recurrence as three
-// launches in a graph loop: P1 1,331 rows 7.3 us (16.3), P1 36k 8.4 (18.9), P1
-// 133k 10.8 (20.7), P1 389k 20.6 (33.3), P2 69k 11.9 (23.4), P2 250k 25.0
-// (37.4), P2 531k 47.5 (58.5), P3 227k 32.2 (52.2); and a solve needs no tuned
+// launches in a graph loop: P1 1,331 rows 6.7 us (16.3), P1 36k 7.9 (18.9), P1
+// 133k 10.4 (20.7), P1 389k 18.5 (33.3), P2 69k 11.3 (23.4), P2 250k 22.5
+// (37.4), P2 531k 38.5 (58.5), P3 227k 30.8 (52.2); and a solve needs no tuned
 // layout, no graph and one host wait: 71 us instead of 180 before the first
 // iteration.  (Measured and left: the rows in one contiguous run per block, as
 // CSR rows of 4 to 16 lanes, as a stream over the entries, or sorted by length:
@@ -40,8 +40,9 @@ struct PcgScalars {
 
 __device__ __forceinline__ bool is_zero(double a) { return fabs(a) < 10.0 * DBL_MIN; }   // utils.h:451
 
+template <int H>
 __global__ void __launch_bounds__(kCoopThreads, 1)
-pcg_coop_kernel(const PcgRun R, int parts) {
+pcg_coop_kernel(const PcgRun R) {
     extern __shared__ double s_vec[];
     __shared__ CoopShared sh;
     __shared__ PcgScalars S;
@@ -49,9 +50,9 @@ pcg_coop_kernel(const PcgRun R, int parts) {
     CoopGrid G(R.exchange, &sh);
     const int t = threadIdx.x;
     const unsigned n = (unsigned)R.A.n;
-    const int m = 32 * (int)((((int64_t)n + 31) / 32 - blockIdx.x + gridDim.x - 1) / gridDim.x);
+    const int m = coop_places(n);
     double *sr = s_vec, *sw = sr + m, *sp = sw + m, *sD = sp + m;   // of the block's places
-    CoopRows L(n, parts, sD + m, &next_unit, R.cols, R.vals);
+    CoopRows<H> L(n, sD + m, &next_unit, R.cols);
     const bool first = blockIdx.x == 0;
 
     // ||b|| and |x|_1 (solver-phg.c:498-518)
@@ -96,11 +97,11 @@ pcg_coop_kernel(const PcgRun R, int parts) {
             if (L.row(i) < n) R.x[L.row(i)] = 0.0;
         return;
     }
-    L.build(R.A);
+    L.build(R.A, [&](int q, double value) { R.vals[q] = value; });
     __syncthreads();
     // r = b - A x, or b when x = 0
     if (S.nonzero) {
-        L.product(R.x, sw);
+        L.template product<false>(R.vals, R.x, sw);
         for (int i = t; i < m; i += kCoopThreads) sr[i] -= sw[i];
     }
     v[0] = v[1] = 0.0;
@@ -134,7 +135,7 @@ pcg_coop_kernel(const PcgRun R, int parts) {
         start = false;
         if (!(ok = G.sync())) break;
         d[0] = 0.0;
-        L.product(R.p, sw);
+        L.template product<false>(R.vals, R.p, sw);
         for (int i = t; i < m; i += kCoopThreads) d[0] += sp[i] * sw[i];
         ok = G.sum(d, [&](const double *s) {
             if (s[0] == 0.0) {
@@ -187,78 +188,25 @@ pcg_coop_kernel(const PcgRun R, int parts) {
     }
 }
 
-struct CoopDevice {
-    int blocks = 0;          // SMs of a device that can launch cooperatively, else 0
-    int64_t smem = 0;        // dynamic shared memory a block may use
-};
-
-CoopDevice coop_device() {
-    CoopDevice d;
-    int dev = 0, coop = 0, sms = 0, smem = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess) {
-        cudaGetLastError();
-        return d;
-    }
-    d.blocks = coop ? (sms < kCoopMaxBlocks ? sms : kCoopMaxBlocks) : 0;
-    d.smem = smem - 4096;   // the kernel's static shared memory
-    return d;
-}
-
-// Shared memory of a block with that many slices: r, w / z, p and the diagonal
-// of each row, and the row bookkeeping.
-constexpr int64_t coop_smem(int64_t slices, int parts) {
-    return slices * 32 * 4 * (int64_t)sizeof(double) + coop_rows_bytes(slices, parts);
-}
-
-// Shared memory a solve takes at most.  What it takes the L1 cache loses, and
-// the product's gathers need that: with 122 KB a block (P2, 531k rows) an
-// iteration takes 47.5 us against 58.5 as separate launches, with 208 KB 71.
-constexpr int64_t kCoopMaxSmem = 136 * 1024;
-// A block per this many entries (a row's vector work counted as four) while
-// there are SMs: below that the barriers of more blocks cost what they save.
-constexpr int64_t kCoopBlockWork = 4096;
-
-// Blocks of a solve; false when it is too large.
-bool coop_split(const CoopDevice &dv, int64_t n, int64_t nnz, int *blocks, int *parts, int64_t *smem) {
-    if (dv.blocks < 1) return false;
-    const int64_t slices = ceil_div(n, 32);
-    int64_t G = ceil_div(nnz + 4 * n, kCoopBlockWork);
-    if (G > slices) G = slices;
-    if (G > dv.blocks) G = dv.blocks;
-    const int64_t per = ceil_div(slices, G);
-    *blocks = (int)G;
-    *parts = coop_parts(per, n, nnz);
-    *smem = coop_smem(per, *parts);
-    return *smem <= dv.smem && *smem <= kCoopMaxSmem;
-}
-
-cudaError_t launch(const PcgRun &R, int blocks, int parts, int64_t smem, cudaStream_t s) {
-    cudaError_t e = cudaFuncSetAttribute(pcg_coop_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    PcgRun run = R;
-    void *args[] = {(void *)&run, (void *)&parts};
-    return cudaLaunchCooperativeKernel((const void *)pcg_coop_kernel, dim3(blocks), dim3(kCoopThreads), args,
-                                       (size_t)smem, s);
-}
+constexpr int64_t kRowBytes = 4 * sizeof(double);   // r, w / z, p, diagonal
 
 }  // namespace
 
 int coop_exchange_doubles() { return kCoopDoubles; }
 
 int64_t pcg_coop_entries(int64_t n, int64_t nnz) {
-    int b, p;
-    int64_t m;
-    return coop_split(coop_device(), n, nnz, &b, &p, &m) ? nnz : -1;
+    CoopSplit sp;
+    return coop_split(n, nnz, kRowBytes, 4, &sp) ? nnz : -1;
 }
 
 cudaError_t launch_pcg_coop(const PcgRun &R, cudaStream_t s) {
-    int blocks, parts;
-    int64_t smem;
-    if (!coop_split(coop_device(), R.A.n, R.nnz, &blocks, &parts, &smem)) return cudaErrorCooperativeLaunchTooLarge;
-    return launch(R, blocks, parts, smem, s);
+    CoopSplit sp;
+    if (!coop_split(R.A.n, R.nnz, kRowBytes, 4, &sp)) return cudaErrorCooperativeLaunchTooLarge;
+    switch (sp.lanes) {
+    case 1: return coop_launch(pcg_coop_kernel<1>, R, sp, s);
+    case 2: return coop_launch(pcg_coop_kernel<2>, R, sp, s);
+    default: return coop_launch(pcg_coop_kernel<4>, R, sp, s);
+    }
 }
 
 }  // namespace phgb

@@ -1,4 +1,4 @@
-"""The solvers that run as one cooperative kernel (FP64 PCG) against the
+"""The solvers that run as one cooperative kernel (FP64 and mixed PCG) against the
 oracle at the edges of their row split: slices of 32 rows that are empty, full
 or part-filled, one block and all of them, rows short and long enough to be
 split among warps, rows too long for the kernel, and a product layout the
@@ -90,3 +90,45 @@ def test_pcg_long_row_and_forced_layout(gpu, oracle):
             its.append(check_pcg(s, oracle, ptr, cols, vals, b, 1e-9))
             assert s.spmv_plan()[:2] == (layout, param)
     assert max(its) - min(its) <= 1
+
+
+@pytest.mark.parametrize("half", [0, 3, 12, 60])
+@pytest.mark.parametrize("n", SIZES)
+def test_mixed_row_split(gpu, oracle, n, half):
+    """The mixed solver on the same splits: the FP64 residual of the iterate it
+    returns, recomputed by the oracle, meets the stopping rule and is the one
+    reported (within the FP64 rounding of a product, 1e-13 of ||b||)."""
+    ptr, cols, vals, b = banded_spd(n, half, seed=n + half)
+    rtol = 1e-9
+    with gpu.Solver(0) as s:
+        s.set_matrix(ptr, cols, vals, b)
+        for x0 in (None, np.linspace(-1.0, 1.0, n)):
+            r0 = b if x0 is None else b - oracle.spmv(ptr, cols, vals, x0)
+            x, nits, res, nupd = s.solve_pcg_mixed(x0=x0, rtol=rtol)
+            r = np.linalg.norm(b - oracle.spmv(ptr, cols, vals, x))
+            slack = 1e-13 * np.linalg.norm(b)
+            assert r <= rtol * np.linalg.norm(r0) + slack
+            assert abs(res - r) <= slack
+            assert nupd >= 1 and nits >= 1
+
+
+def test_mixed_long_row_forced_layout_maxit(gpu, oracle):
+    ptr, cols, vals, b = banded_spd(1500, 4, seed=5, long_row=True)
+    with gpu.Solver(0) as s:
+        s.set_matrix(ptr, cols, vals, b)
+        x, nits, res, _ = s.solve_pcg_mixed(rtol=1e-9)
+        assert np.linalg.norm(b - oracle.spmv(ptr, cols, vals, x)) <= 1e-9 * np.linalg.norm(b) * (1 + 1e-6)
+    ptr, cols, vals, b = banded_spd(3000, 12, seed=6)
+    with gpu.Solver(0) as s:
+        s.set_matrix(ptr, cols, vals, b)
+        x0, n0, _, _ = s.solve_pcg_mixed(rtol=1e-9)
+        assert s.spmv_plan()[2]["fp32_unroll"] > 0
+        for maxit in (0, 1, 3):
+            x, nits, res, _ = s.solve_pcg_mixed(rtol=1e-12, maxit=maxit)
+            assert nits == maxit
+            r = np.linalg.norm(b - oracle.spmv(ptr, cols, vals, x))
+            assert abs(res - r) <= 1e-13 * np.linalg.norm(b)
+        s.set_spmv_plan32("pair", 4)
+        x1, n1, _, _ = s.solve_pcg_mixed(rtol=1e-9)
+        assert s.spmv_plan()[2]["fp32_layout"] == "pair"
+        assert abs(n1 - n0) <= 2
