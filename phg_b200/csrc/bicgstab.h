@@ -20,6 +20,8 @@ enum {
     BICG_SMALL_S = 2,      // ||s|| <= 1e-60: x += alpha p^, residual recomputed (host)
     BICG_BREAKDOWN = 3,    // rh.v = 0 or t.t = 0 (the reference would divide by zero)
     BICG_NONFINITE = 4,
+    BICG_PASS_LIMIT = 13,  // a barrier of the one-kernel solve gave up
+    BICG_DECLINED = 15,    // the one-kernel solve does not take the matrix
 };
 
 struct BicgBuffers {

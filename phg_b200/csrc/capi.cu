@@ -13,6 +13,7 @@
 #include "gmres.h"
 #include "mixed.h"
 #include "mixed_coop.h"
+#include "krylov_coop.h"
 #include "pcg_coop.h"
 
 #include <math.h>
@@ -693,6 +694,15 @@ SpmvPlan make_plan(phgGpuSystem *s, int kind, int param) {
     return P;
 }
 
+// Memory of a one-kernel solve's matrix copy and exchange.
+int coop_buffers(phgGpuSystem *s, int64_t entries) {
+    CHECK_RC(s->coop_cols.ensure((size_t)entries));
+    CHECK_RC(s->coop_vals.ensure((size_t)entries));
+    CHECK_RC(s->coop_xch.ensure((size_t)coop_exchange_doubles()));
+    CK(cudaMemsetAsync(s->coop_xch.p, 0, sizeof(double) * coop_exchange_doubles(), s->stream));
+    return PHG_GPU_OK;
+}
+
 // Whether the caller chose the product layout for the current matrix shape.
 bool plan_forced(const phgGpuSystem *s) {
     return s->plan_set && s->tuned && s->tuned_n == s->n && s->tuned_nnz == s->nnz;
@@ -1323,14 +1333,11 @@ static int mixed_one_kernel(phgGpuSystem *s, double rtol, double btol, double at
     if (s->plan32_set && s->unroll32 != 0 && s->tuned32_n == n && s->tuned32_nnz == s->nnz) return 0;
     const int64_t entries = mixed_coop_entries(n, s->nnz);
     if (entries < 0) return 0;
-    CHECK_RC(s->coop_cols.ensure((size_t)entries));
-    CHECK_RC(s->coop_vals.ensure((size_t)entries));
+    CHECK_RC(coop_buffers(s, entries));
     CHECK_RC(s->coop_vals32.ensure((size_t)entries));
-    CHECK_RC(s->coop_xch.ensure((size_t)coop_exchange_doubles()));
     CHECK_RC(s->u32.ensure((size_t)n));
     CHECK_RC(s->mixed_out.ensure(1));
     if (s->h_mixed == nullptr) CK(cudaMallocHost((void **)&s->h_mixed, sizeof(MixedResult)));
-    CK(cudaMemsetAsync(s->coop_xch.p, 0, sizeof(double) * coop_exchange_doubles(), s->stream));
     const MixedRun run{CsrView{n, s->rp.p, s->ci.p, s->va.p}, s->nnz, s->coop_cols.p, s->coop_vals32.p, s->coop_vals.p,
                        s->x.p, s->u32.p, s->rhs.p, s->diag.p, rtol, btol, atol, 0.1, maxit, s->coop_xch.p,
                        s->mixed_out.p};
@@ -1661,10 +1668,7 @@ int pcg_one_kernel(phgGpuSystem *s, const double *drhs, double rtol, double btol
     if (plan_forced(s)) return 0;
     const int64_t entries = pcg_coop_entries(n, s->nnz);
     if (entries < 0) return 0;
-    CHECK_RC(s->coop_cols.ensure((size_t)entries));
-    CHECK_RC(s->coop_vals.ensure((size_t)entries));
-    CHECK_RC(s->coop_xch.ensure((size_t)coop_exchange_doubles()));
-    CK(cudaMemsetAsync(s->coop_xch.p, 0, sizeof(double) * coop_exchange_doubles(), s->stream));
+    CHECK_RC(coop_buffers(s, entries));
     const PcgRun run{CsrView{n, s->rp.p, s->ci.p, s->va.p}, s->nnz, s->coop_cols.p, s->coop_vals.p, s->x.p, s->p.p,
                      drhs, s->diag.p, rtol, btol, atol, maxit, dhist, s->coop_xch.p, s->st.p};
     CK(launch_pcg_coop(run, s->stream));
@@ -1785,12 +1789,50 @@ int pcg_core(phgGpuSystem *s, const double *drhs, double rtol, double btol, doub
     return nits;
 }
 
+// BiCGstab as one cooperative kernel on s->x, its state in s->h_bst.  Returns 1,
+// or 0 when the kernel does not take it (as pcg_one_kernel).
+int bicg_one_kernel(phgGpuSystem *s, double rtol, double btol, double atol, int maxit, double *dhist) {
+    const int64_t n = s->n;
+    const int64_t entries = plan_forced(s) ? -1 : bicg_coop_entries(n, s->nnz);
+    if (entries < 0) return 0;
+    CHECK_RC(coop_buffers(s, entries));
+    CHECK_RC(s->bicg_st.ensure(1));
+    if (s->h_bst == nullptr) CK(cudaMallocHost((void **)&s->h_bst, sizeof(BicgState)));
+    const BicgRun run{CsrView{n, s->rp.p, s->ci.p, s->va.p}, s->nnz, s->coop_cols.p, s->coop_vals.p, s->x.p, s->p.p,
+                      s->Ap.p, s->rhs.p, s->diag.p, rtol, btol, atol, maxit, dhist, s->coop_xch.p, s->bicg_st.p};
+    CK(launch_bicg_coop(run, s->stream));
+    s->launches += 1;
+    CK(cudaMemcpyAsync(s->h_bst, s->bicg_st.p, sizeof(BicgState), cudaMemcpyDeviceToHost, s->stream));
+    CK(cudaStreamSynchronize(s->stream));
+    if (s->h_bst->status == BICG_DECLINED) return 0;
+    s->plan_due = true;
+    return 1;
+}
+
+// What a BiCGstab solve returns for the state in s->h_bst.
+int bicg_result(phgGpuSystem *s) {
+    const int nits = s->h_bst->nits;
+    switch (s->h_bst->status) {
+    case BICG_BREAKDOWN:
+        return fail(PHG_GPU_ERR_BREAKDOWN, "BiCGstab breakdown after %d iterations (rh.v = 0 or t.t = 0)", nits);
+    case BICG_NONFINITE: return fail(PHG_GPU_ERR_NAN, "BiCGstab: non-finite values after %d iterations", nits);
+    case BICG_PASS_LIMIT: return fail(PHG_GPU_ERR_STATE, "BiCGstab: the iteration loop exceeded its bound");
+    default: return nits;
+    }
+}
+
 // BiCGstab with the Jacobi preconditioner (solver_BiCGstab,
 // solver-phg.c:606-781) from the initial guess in s->x.
 int bicg_core(phgGpuSystem *s, double rtol, double btol, double atol, int maxit, double *dhist,
               double *residual) {
     const int64_t n = s->n;
     const double *drhs = s->rhs.p;
+    const int one = bicg_one_kernel(s, rtol, btol, atol, maxit, dhist);
+    if (one < 0) return one;
+    if (one > 0) {
+        if (residual) *residual = s->h_bst->residual;
+        return bicg_result(s);
+    }
     CK(cudaMemsetAsync(s->ticket.p, 0, sizeof(unsigned) * kRedTickets, s->stream));
     CK(launch_init_sums(n, 0, s->x.p, drhs, s->diag.p, s->partials.p, s->ticket.p, s->sums.p, s->stream));
     s->launches += 1;
@@ -1879,11 +1921,7 @@ int bicg_core(phgGpuSystem *s, double rtol, double btol, double atol, int maxit,
                                s->stream));
     }
     if (residual) *residual = res;
-    if (s->h_bst->status == BICG_BREAKDOWN)
-        return fail(PHG_GPU_ERR_BREAKDOWN, "BiCGstab breakdown after %d iterations (rh.v = 0 or t.t = 0)", nits);
-    if (s->h_bst->status == BICG_NONFINITE)
-        return fail(PHG_GPU_ERR_NAN, "BiCGstab: non-finite values after %d iterations", nits);
-    return nits;
+    return bicg_result(s);
 }
 
 }  // namespace
@@ -1929,6 +1967,40 @@ static int gmres_impl(phgGpuSystem *s, int restart, int augk, double rtol, doubl
     CHECK_RC(solver_buffers(s));
     const int64_t n = s->n;
     CHECK_RC(copy_in(s, s->x.p, x, (size_t)n));
+    const int64_t stride = bicg_stride(n);
+    // z, V_0..V_(R+1); FLGMRES_r also F_0..F_R and Z_0..Z_(augk-1)
+    const int nvec = (restart + 3) + (flex ? (restart + 1) + augk : 0);
+    CHECK_RC(s->gm_st.ensure(1));
+    if (s->h_gst == nullptr) CK(cudaMallocHost((void **)&s->h_gst, sizeof(GmresState)));
+    // as one cooperative kernel, unless it does not take the matrix (as pcg_one_kernel)
+    const int64_t entries = plan_forced(s) ? -1 : gmres_coop_entries(n, s->nnz, restart);
+    if (entries >= 0) {
+        CHECK_RC(coop_buffers(s, entries));
+        CHECK_RC(s->gm_vecs.ensure((size_t)stride * nvec));
+        double *V = s->gm_vecs.p + stride, *F1 = flex ? s->gm_vecs.p + (int64_t)(restart + 3) * stride : nullptr;
+        double *Z1 = flex ? F1 + (int64_t)(restart + 1) * stride : nullptr;
+        if (flex) CK(cudaMemsetAsync(Z1, 0, sizeof(double) * (size_t)stride * augk, s->stream));
+        const GmresRun run{CsrView{n, s->rp.p, s->ci.p, s->va.p}, s->nnz, s->coop_cols.p, s->coop_vals.p, s->x.p, s->rhs.p,
+                           s->diag.p, V, F1, Z1, stride, rtol, btol, atol, maxit, mk, flex ? augk : -1, s->coop_xch.p,
+                           s->gm_st.p};
+        CK(launch_gmres_coop(run, s->stream));
+        s->launches += 1;
+        CK(cudaMemcpyAsync(s->h_gst, s->gm_st.p, sizeof(GmresState), cudaMemcpyDeviceToHost, s->stream));
+        CK(cudaStreamSynchronize(s->stream));
+        const GmresState &g = *s->h_gst;
+        if (g.status != kStatusDeclined) {
+            s->plan_due = true;
+            if (residual) *residual = g.residual;
+            if (g.status == GMRES_NONFINITE)
+                return fail(PHG_GPU_ERR_NAN, "GMRES: non-finite values after %d iterations", g.nits);
+            if (g.status == kStatusPassLimit)
+                return fail(PHG_GPU_ERR_STATE, "GMRES: the iteration loop exceeded its bound");
+            const int nits = g.nits;
+            CHECK_RC(copy_out(s, x, s->x.p, (size_t)n));
+            CK(cudaStreamSynchronize(s->stream));
+            return nits;
+        }
+    }
     // ||b|| (solver-phg.c:1071-1075)
     CK(cudaMemsetAsync(s->ticket.p, 0, sizeof(unsigned) * kRedTickets, s->stream));
     CK(launch_init_sums(n, 0, s->x.p, s->rhs.p, s->diag.p, s->partials.p, s->ticket.p, s->sums.p, s->stream));
@@ -1944,13 +2016,8 @@ static int gmres_impl(phgGpuSystem *s, int restart, int augk, double rtol, doubl
         return 0;
     }
     CHECK_RC(tune_spmv(s));
-    const int64_t stride = bicg_stride(n);
-    // z, V_0..V_(R+1); FLGMRES_r also F_0..F_R and Z_0..Z_(augk-1)
-    const int nvec = (restart + 3) + (flex ? (restart + 1) + augk : 0);
     CHECK_RC(s->gm_vecs.ensure((size_t)stride * nvec));
     CHECK_RC(s->gm_small.ensure((size_t)gmres_small_doubles(restart)));
-    CHECK_RC(s->gm_st.ensure(1));
-    if (s->h_gst == nullptr) CK(cudaMallocHost((void **)&s->h_gst, sizeof(GmresState)));
     const int R2 = restart + 2;
     GmresState init{};
     init.rtol = rtol;

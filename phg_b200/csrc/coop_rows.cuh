@@ -251,8 +251,8 @@ inline int coop_lanes(int64_t slices, int64_t n, int64_t nnz, int most) {
 }
 
 // The launch of a one-kernel solver: blocks, lanes a row and shared memory
-// (`row_bytes` of vectors a row, and the row bookkeeping); false when it is too
-// large.
+// (`fixed_bytes`, `row_bytes` of vectors a row, and the row bookkeeping); false
+// when it is too large.
 //
 // Shared memory a solve takes at most: what it takes the L1 cache loses, and
 // the product's gathers need that.  With 122 KB a block (P2, 531k rows) an
@@ -268,7 +268,8 @@ struct CoopSplit {
     int64_t smem = 0;
 };
 
-inline bool coop_split(int64_t n, int64_t nnz, int64_t row_bytes, int most_lanes, CoopSplit *out) {
+inline bool coop_split(int64_t n, int64_t nnz, int64_t row_bytes, int64_t fixed_bytes, int most_lanes,
+                       CoopSplit *out) {
     int dev = 0, coop = 0, sms = 0, most = 0;
     if (cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess ||
@@ -286,7 +287,7 @@ inline bool coop_split(int64_t n, int64_t nnz, int64_t row_bytes, int most_lanes
     const int64_t per = ceil_div(slices, G);
     out->blocks = (int)G;
     out->lanes = coop_lanes(per, n, nnz, most_lanes);
-    out->smem = 32 * per * row_bytes + coop_rows_bytes(per, out->lanes);
+    out->smem = fixed_bytes + 32 * per * row_bytes + coop_rows_bytes(per, out->lanes);
     return out->smem <= kCoopMaxSmem && out->smem <= most - 4096;   // 4 KB of static shared memory at most
 }
 

@@ -196,12 +196,12 @@ int coop_exchange_doubles() { return kCoopDoubles; }
 
 int64_t pcg_coop_entries(int64_t n, int64_t nnz) {
     CoopSplit sp;
-    return coop_split(n, nnz, kRowBytes, 4, &sp) ? nnz : -1;
+    return coop_split(n, nnz, kRowBytes, 0, 4, &sp) ? nnz : -1;
 }
 
 cudaError_t launch_pcg_coop(const PcgRun &R, cudaStream_t s) {
     CoopSplit sp;
-    if (!coop_split(R.A.n, R.nnz, kRowBytes, 4, &sp)) return cudaErrorCooperativeLaunchTooLarge;
+    if (!coop_split(R.A.n, R.nnz, kRowBytes, 0, 4, &sp)) return cudaErrorCooperativeLaunchTooLarge;
     switch (sp.lanes) {
     case 1: return coop_launch(pcg_coop_kernel<1>, R, sp, s);
     case 2: return coop_launch(pcg_coop_kernel<2>, R, sp, s);

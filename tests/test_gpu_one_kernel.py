@@ -1,4 +1,5 @@
-"""The solvers that run as one cooperative kernel (FP64 and mixed PCG) against the
+"""The solvers that run as one cooperative kernel (PCG, mixed PCG, BiCGstab, GMRES)
+against the
 oracle at the edges of their row split: slices of 32 rows that are empty, full
 or part-filled, one block and all of them, rows short and long enough to be
 split among warps, rows too long for the kernel, and a product layout the
@@ -132,3 +133,35 @@ def test_mixed_long_row_forced_layout_maxit(gpu, oracle):
         x1, n1, _, _ = s.solve_pcg_mixed(rtol=1e-9)
         assert s.spmv_plan()[2]["fp32_layout"] == "pair"
         assert abs(n1 - n0) <= 2
+
+
+@pytest.mark.parametrize("half", [3, 12, 60])
+@pytest.mark.parametrize("n", SIZES)
+def test_nonsymmetric_row_split(gpu, oracle, n, half):
+    """BiCGstab, GMRES_r and FLGMRES_r on the same splits, the couplings to
+    later rows halved so that the matrix is not symmetric.  The residuals are
+    recomputed by the oracle; GMRES's estimate and BiCGstab's recurrence drift
+    from them by rounding only (1e-6 of the tolerance at these condition
+    numbers)."""
+    ptr, cols, vals, b = banded_spd(n, half, seed=n + half)
+    rows = np.repeat(np.arange(n), np.diff(ptr))
+    vals = np.where(cols > rows, 0.5 * vals, vals)
+    diag = diagonal(ptr, cols, vals)
+    rtol, nb = 1e-9, np.linalg.norm(b)
+    kw = dict(rtol=rtol, btol=0.0, atol=0.0)
+    with gpu.Solver(0) as s:
+        s.set_matrix(ptr, cols, vals, b)
+        xo, no = oracle.bicgstab(ptr, cols, vals, diag, b, **kw)[:2]
+        x, nits, res, hist = s.solve_bicgstab(history=True, **kw)
+        assert abs(nits - no) <= 2 and len(hist) == nits + 1 and hist[-1] == res
+        assert np.linalg.norm(b - oracle.spmv(ptr, cols, vals, x)) <= rtol * nb * (1 + 1e-6)
+        assert np.linalg.norm(x - xo) <= 1e3 * rtol * np.linalg.norm(xo)
+        for x0 in (None, np.linspace(-1.0, 1.0, n)):
+            xo, no = oracle.gmres(ptr, cols, vals, diag, b, restart=6, x0=x0, **kw)[:2]
+            x, nits, _ = s.solve_gmres(restart=6, x0=x0, **kw)
+            assert abs(nits - no) <= 2
+            assert np.linalg.norm(x - xo) <= 1e3 * rtol * np.linalg.norm(xo)
+            xo, no = oracle.flgmres(ptr, cols, vals, diag, b, restart=4, augk=2, x0=x0, **kw)[:2]
+            x, nits, _ = s.solve_flgmres(restart=4, augk=2, x0=x0, **kw)
+            assert abs(nits - no) <= 2
+            assert np.linalg.norm(x - xo) <= 1e3 * rtol * np.linalg.norm(xo)
