@@ -24,6 +24,8 @@
 #include "common.cuh"
 #include "assemble.h"
 
+#include <limits.h>
+
 namespace phgb {
 
 // ---------------------------------------------------------------------------
@@ -108,7 +110,10 @@ __device__ __forceinline__ void jacobian_vol(const double *x, double *J, double 
 //           plus, when c = mass != 0, c times the mass matrix, integral of
 //           phi_b phi_a with the order-2p rule (phgQuadBasABas with A = NULL,
 //           quad.c:5582-5625), added as stiffness + c * mass the way
-//           examples/simplest.c:68-72 writes the element matrix
+//           examples/simplest.c:68-72 writes the element matrix; the sums over
+//           the points do not depend on the element and come from a table (mt)
+//           made with the same operations (summed per entry, they made the P2
+//           element kernel of a time step 1.7 times slower)
 //   Re[e]   N right-hand side entries, integral of f_h phi_a with the order-2p
 //           rule (phgQuadDofTimesBas, quad.c:5481-5530; f_h at the points as
 //           phgDofEval_, dof-utils.c:59-300)
@@ -138,44 +143,61 @@ __device__ const unsigned char g_pair_a[210] = {
 };
 
 // Geometry: one thread per element, J (16) and the volume into geo[e][0..16].
-__global__ void __launch_bounds__(128)
+// A block's results go through shared memory, so that its stores are one
+// contiguous run (a thread storing its own 136 bytes touches a sector a lane
+// and store: 262 against 85 us for 2 million elements).
+constexpr int kGeoThreads = 128;
+
+__global__ void __launch_bounds__(kGeoThreads)
 geometry_kernel(int64_t nelem, int64_t nvert, const double *__restrict__ verts, const int32_t *__restrict__ elems,
                 double *__restrict__ geo, int *status) {
-    for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < nelem; e += (int64_t)gridDim.x * blockDim.x) {
-        double x[12];
-        bool ok = true;
+    __shared__ double s_geo[kGeoThreads * 17];
+    for (int64_t e0 = (int64_t)blockIdx.x * kGeoThreads; e0 < nelem; e0 += (int64_t)gridDim.x * kGeoThreads) {
+        const int64_t e = e0 + threadIdx.x;
+        if (e < nelem) {
+            double x[12];
+            bool ok = true;
+            const int4 ev = __ldg(reinterpret_cast<const int4 *>(elems) + e);
+            const int32_t vs[4] = {ev.x, ev.y, ev.z, ev.w};
 #pragma unroll
-        for (int j = 0; j < 4; j++) {
-            const int32_t v = elems[4 * e + j];
-            if (v < 0 || v >= nvert) {
-                ok = false;
-                x[3 * j] = x[3 * j + 1] = x[3 * j + 2] = 0.0;
-            } else {
-                x[3 * j] = verts[3 * (int64_t)v];
-                x[3 * j + 1] = verts[3 * (int64_t)v + 1];
-                x[3 * j + 2] = verts[3 * (int64_t)v + 2];
+            for (int j = 0; j < 4; j++) {
+                const int32_t v = vs[j];
+                if (v < 0 || v >= nvert) {
+                    ok = false;
+                    x[3 * j] = x[3 * j + 1] = x[3 * j + 2] = 0.0;
+                } else {
+                    x[3 * j] = verts[3 * (int64_t)v];
+                    x[3 * j + 1] = verts[3 * (int64_t)v + 1];
+                    x[3 * j + 2] = verts[3 * (int64_t)v + 2];
+                }
             }
+            if (!ok) atomicExch(status, PHGB_DEV_BAD_INDEX);
+            bool fin = true;
+#pragma unroll
+            for (int t = 0; t < 12; t++) fin = fin && isfinite(x[t]);
+            if (!fin) atomicExch(status, PHGB_DEV_NONFINITE);
+            double J[16], vol;
+            jacobian_vol(x, J, vol);
+            double *o = s_geo + threadIdx.x * 17;
+#pragma unroll
+            for (int t = 0; t < 16; t++) o[t] = J[t];
+            o[16] = vol;
         }
-        if (!ok) atomicExch(status, PHGB_DEV_BAD_INDEX);
-        bool fin = true;
-#pragma unroll
-        for (int t = 0; t < 12; t++) fin = fin && isfinite(x[t]);
-        if (!fin) atomicExch(status, PHGB_DEV_NONFINITE);
-        double J[16], vol;
-        jacobian_vol(x, J, vol);
-        double *o = geo + (size_t)e * kGeo;
-#pragma unroll
-        for (int t = 0; t < 16; t++) o[t] = J[t];
-        o[16] = vol;
+        __syncthreads();
+        const int count = (int)(nelem - e0 < kGeoThreads ? nelem - e0 : kGeoThreads) * kGeo;
+        for (int q = threadIdx.x; q < count; q += kGeoThreads) {
+            const int t = q / kGeo, i = q - t * kGeo;
+            geo[(size_t)e0 * kGeo + q] = i < 17 ? s_geo[t * 17 + i] : 0.0;
+        }
+        __syncthreads();
     }
 }
 
-// Quadrature weights, passed by value: every lane reads the same weight at
+// Stiffness weights, passed by value: every lane reads the same weight at
 // the same time, so they are read from the kernel's parameter (constant)
 // bank instead of through the load/store pipe the kernel is bound by.
 struct ElemWeights {
     double wk[kElemMaxQK];
-    double wr[kElemMaxQR];
 };
 
 // Element matrices and vectors: one warp per element.
@@ -183,8 +205,8 @@ template <int P>
 __global__ void __launch_bounds__(ElemDims<P>::WARPS * 32)
 element_kernel(int64_t nelem, int64_t ndof, const double *__restrict__ geo, const int32_t *__restrict__ e2l,
                const double *__restrict__ kappa, const double mass, const double *__restrict__ f,
-               const ElemWeights Wt, const double *__restrict__ gk, const double *__restrict__ br,
-               const double *__restrict__ brt,
+               const ElemWeights Wt, const double *__restrict__ gk, const double *__restrict__ mt,
+               const double *__restrict__ bw, const double *__restrict__ brt,
                double *__restrict__ Ke, double *__restrict__ Re, int *status) {
     using D = ElemDims<P>;
     constexpr int N = D::N, QK = D::QK, QR = D::QR, W = D::WARPS;
@@ -264,20 +286,13 @@ element_kernel(int64_t nelem, int64_t ndof, const double *__restrict__ geo, cons
                 d = rn_add(d, kappa != nullptr ? rn_mul(t, kap) : t);
             }
             double v = rn_mul(d, vol);
-            if (mass != 0.0) {
-                double dm = 0.;
-                for (int q = 0; q < QR; q++) {
-                    const double d0 = rn_add(0., rn_mul(br[q * N + b], br[q * N + a]));
-                    dm = rn_add(dm, rn_mul(d0, Wt.wr[q]));
-                }
-                v = rn_add(v, rn_mul(mass, rn_mul(dm, vol)));
-            }
+            if (mass != 0.0) v = rn_add(v, rn_mul(mass, rn_mul(__ldg(&mt[a * N + b]), vol)));
             K[a * N + b] = v;
             K[b * N + a] = v;
         }
         if (lane < N) {
             double d = 0.0;
-            for (int q = 0; q < QR; q++) d = rn_add(d, rn_mul(rn_mul(br[q * N + lane], Wt.wr[q]), fq[q]));
+            for (int q = 0; q < QR; q++) d = rn_add(d, rn_mul(bw[q * N + lane], fq[q]));
             Re[(size_t)e * N + lane] = rn_mul(d, vol);
         }
         __syncwarp();
@@ -306,8 +321,8 @@ template <int P>
 __global__ void __launch_bounds__(128, 6)   // 80 registers: 24 warps an SM (96 without the bound: 20)
 element_lanes_kernel(int64_t nelem, int64_t ndof, const double *__restrict__ geo, const int32_t *__restrict__ e2l,
                      const double *__restrict__ kappa, const double mass, const double *__restrict__ f,
-                     const ElemWeights Wt, const double *__restrict__ gk, const double *__restrict__ br,
-                     const double *__restrict__ brt, double *__restrict__ Ke, double *__restrict__ Re, int *status) {
+                     const ElemWeights Wt, const double *__restrict__ gk, const double *__restrict__ mt,
+                     const double *__restrict__ bw, const double *__restrict__ brt, double *__restrict__ Ke, double *__restrict__ Re, int *status) {
     using D = ElemDims<P>;
     constexpr int N = D::N, QK = D::QK, QR = D::QR, W = 4;
     constexpr int EPW = 32 / N;                  // elements per warp
@@ -404,19 +419,12 @@ element_lanes_kernel(int64_t nelem, int64_t ndof, const double *__restrict__ geo
                 d = rn_add(d, kappa != nullptr ? rn_mul(t, kap) : t);
             }
             double v = rn_mul(d, vol);
-            if (mass != 0.0) {
-                double dm = 0.;
-                for (int q = 0; q < QR; q++) {
-                    const double d0 = rn_add(0., rn_mul(br[q * N + b], br[q * N + a]));
-                    dm = rn_add(dm, rn_mul(d0, Wt.wr[q]));
-                }
-                v = rn_add(v, rn_mul(mass, rn_mul(dm, vol)));
-            }
+            if (mass != 0.0) v = rn_add(v, rn_mul(mass, rn_mul(__ldg(&mt[a * N + b]), vol)));
             if (act) Ke[((size_t)e * N + a) * N + b] = v;
         }
         if (act) {
             double d = 0.0;
-            for (int q = 0; q < QR; q++) d = rn_add(d, rn_mul(rn_mul(br[q * N + b], Wt.wr[q]), fq[q]));
+            for (int q = 0; q < QR; q++) d = rn_add(d, rn_mul(bw[q * N + b], fq[q]));
             Re[(size_t)e * N + b] = rn_mul(d, vol);
         }
         __syncwarp();
@@ -435,8 +443,8 @@ template <int P>
 __global__ void __launch_bounds__(128, 4)   // 128 registers, no spills (5 blocks: 96 registers, 1% slower)
 element_cols2_kernel(int64_t nelem, int64_t ndof, const double *__restrict__ geo, const int32_t *__restrict__ e2l,
                      const double *__restrict__ kappa, const double mass, const double *__restrict__ f,
-                     const ElemWeights Wt, const double *__restrict__ gk, const double *__restrict__ br,
-                     const double *__restrict__ brt, double *__restrict__ Ke, double *__restrict__ Re, int *status) {
+                     const ElemWeights Wt, const double *__restrict__ gk, const double *__restrict__ mt,
+                     const double *__restrict__ bw, const double *__restrict__ brt, double *__restrict__ Ke, double *__restrict__ Re, int *status) {
     using D = ElemDims<P>;
     constexpr int N = D::N, QK = D::QK, QR = D::QR, W = 4, H = N / 2;
     static_assert(N % 2 == 0, "columns are paired");
@@ -546,14 +554,8 @@ element_cols2_kernel(int64_t nelem, int64_t ndof, const double *__restrict__ geo
             }
             double v1 = rn_mul(d1, vol), v2 = rn_mul(d2, vol);
             if (mass != 0.0) {
-                double m1 = 0., m2 = 0.;
-                for (int q = 0; q < QR; q++) {
-                    const double ba = br[q * N + a];
-                    m1 = rn_add(m1, rn_mul(rn_mul(br[q * N + b1], ba), Wt.wr[q]));
-                    m2 = rn_add(m2, rn_mul(rn_mul(br[q * N + b2], ba), Wt.wr[q]));
-                }
-                v1 = rn_add(v1, rn_mul(mass, rn_mul(m1, vol)));
-                v2 = rn_add(v2, rn_mul(mass, rn_mul(m2, vol)));
+                v1 = rn_add(v1, rn_mul(mass, rn_mul(__ldg(&mt[a * N + b1]), vol)));
+                v2 = rn_add(v2, rn_mul(mass, rn_mul(__ldg(&mt[a * N + b2]), vol)));
             }
             if (act) {
                 Ke_e[a * N + b1] = v1;
@@ -563,8 +565,8 @@ element_cols2_kernel(int64_t nelem, int64_t ndof, const double *__restrict__ geo
         if (act) {
             double r1 = 0.0, r2 = 0.0;
             for (int q = 0; q < QR; q++) {
-                r1 = rn_add(r1, rn_mul(rn_mul(br[q * N + b1], Wt.wr[q]), fq[q]));
-                r2 = rn_add(r2, rn_mul(rn_mul(br[q * N + b2], Wt.wr[q]), fq[q]));
+                r1 = rn_add(r1, rn_mul(bw[q * N + b1], fq[q]));
+                r2 = rn_add(r2, rn_mul(bw[q * N + b2], fq[q]));
             }
             Re[(size_t)e * N + b1] = rn_mul(r1, vol);
             Re[(size_t)e * N + b2] = rn_mul(r2, vol);
@@ -598,19 +600,51 @@ __global__ void inc_fill_kernel(int64_t nkeys, int64_t ndof, const int32_t *__re
     }
 }
 
-// Sorts each DOF's short incidence list ascending (element order).
-__global__ void inc_sort_kernel(int64_t ndof, const int32_t *__restrict__ inc_ptr,
-                                int32_t *__restrict__ inc) {
-    for (int64_t d = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; d < ndof;
-         d += (int64_t)gridDim.x * blockDim.x) {
-        const int32_t b = inc_ptr[d], n = inc_ptr[d + 1] - b;
+// Sorts each DOF's incidence list ascending (element order).  Eight lanes take
+// a DOF, up to four keys each in registers, and find every key's place by
+// counting the smaller ones; lists over 32 keys are sorted in place by one
+// lane.  (A lane per DOF sorting in memory took 258 us for 357,911 P1 DOFs of 24
+// keys, this 42.)
+__global__ void inc_sort_kernel(int64_t ndof, const int32_t *__restrict__ inc_ptr, int32_t *__restrict__ inc) {
+    constexpr int L = 8, Q = 4;
+    const int gl = threadIdx.x % L;
+    const int64_t step = (int64_t)gridDim.x * blockDim.x / L;
+    // uniform bound: every lane of a warp reaches the shuffles
+    for (int64_t base = ((int64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31)) / L; base < ndof; base += step) {
+        const int64_t d = base + (threadIdx.x & 31) / L;
+        const int32_t b = d < ndof ? inc_ptr[d] : 0, n = d < ndof ? inc_ptr[d + 1] - b : 0;
         int32_t *v = inc + b;
-        for (int i = 1; i < n; i++) {
-            const int32_t key = v[i];
-            int j = i - 1;
-            while (j >= 0 && v[j] > key) { v[j + 1] = v[j]; j--; }
-            v[j + 1] = key;
+        const int m = n <= L * Q ? n : 0;
+        int32_t key[Q];
+        int place[Q];
+#pragma unroll
+        for (int q = 0; q < Q; q++) {
+            key[q] = gl + L * q < m ? v[gl + L * q] : INT_MAX;
+            place[q] = 0;
         }
+        const int most = __reduce_max_sync(0xffffffffu, (unsigned)m);
+#pragma unroll
+        for (int p = 0; p < Q; p++) {
+            if (L * p >= most) break;
+#pragma unroll
+            for (int j = 0; j < L; j++) {
+                const int32_t other = __shfl_sync(0xffffffffu, key[p], j, L);
+#pragma unroll
+                for (int q = 0; q < Q; q++) place[q] += other < key[q];
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < Q; q++)
+            if (gl + L * q < m) v[place[q]] = key[q];
+        if (n > L * Q && gl == 0) {
+            for (int i = 1; i < n; i++) {
+                const int32_t k = v[i];
+                int j = i - 1;
+                while (j >= 0 && v[j] > k) { v[j + 1] = v[j]; j--; }
+                v[j + 1] = k;
+            }
+        }
+        __syncwarp();
     }
 }
 
@@ -618,47 +652,87 @@ __global__ void inc_sort_kernel(int64_t ndof, const int32_t *__restrict__ inc_pt
 // Exclusive scan of int32 counts (three phases), with the total.
 constexpr int kScanBlock = 1024;
 
-__global__ void scan_local_kernel(int64_t n, const int32_t *__restrict__ in, int32_t *__restrict__ out,
-                                  int64_t *__restrict__ block_sums) {
-    __shared__ int64_t s[kScanBlock];
-    const int64_t i = (int64_t)blockIdx.x * kScanBlock + threadIdx.x;
-    const int64_t v = i < n ? in[i] : 0;
-    s[threadIdx.x] = v;
+// Inclusive sum over the block's threads (1024 of them).
+__device__ __forceinline__ int64_t block_scan(int64_t v) {
+    __shared__ int64_t s_warp[32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    auto warp_scan = [lane](int64_t a) {
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int64_t t = __shfl_up_sync(0xffffffffu, a, o);
+            if (lane >= o) a += t;
+        }
+        return a;
+    };
+    v = warp_scan(v);
+    if (lane == 31) s_warp[w] = v;
     __syncthreads();
-    for (int o = 1; o < kScanBlock; o <<= 1) {
-        const int64_t t = threadIdx.x >= o ? s[threadIdx.x - o] : 0;
-        __syncthreads();
-        s[threadIdx.x] += t;
-        __syncthreads();
-    }
-    if (i < n) out[i] = (int32_t)(s[threadIdx.x] - v);   // block-local exclusive
-    if (threadIdx.x == kScanBlock - 1) block_sums[blockIdx.x] = s[threadIdx.x];
+    if (w == 0) s_warp[lane] = warp_scan(s_warp[lane]);
+    __syncthreads();
+    return v + (w > 0 ? s_warp[w - 1] : 0);
 }
 
-__global__ void scan_blocks_kernel(int64_t nb, int64_t *__restrict__ block_sums, int64_t *__restrict__ total) {
-    // single block: serial per thread chunk, then across threads
-    __shared__ int64_t s[1024];
+// One or two arrays of the same length scanned by the same launches
+// (blockIdx.y picks one): out[0..n] = exclusive prefix sums of in[0..n-1], out[n]
+// the total.  ws holds ceil((n + 1) / kScanBlock) + 1 words per array.
+struct ScanPair {
+    const int32_t *in[2];
+    int32_t *out[2];
+    int64_t *ws[2];
+};
+
+__global__ void __launch_bounds__(kScanBlock)
+scan_local_kernel(int64_t n, const ScanPair S) {
+    const int64_t i = (int64_t)blockIdx.x * kScanBlock + threadIdx.x;
+    const int64_t v = i < n ? S.in[blockIdx.y][i] : 0;
+    const int64_t s = block_scan(v);
+    if (i < n) S.out[blockIdx.y][i] = (int32_t)(s - v);   // block-local exclusive
+    if (threadIdx.x == kScanBlock - 1) S.ws[blockIdx.y][blockIdx.x] = s;
+}
+
+// One block an array: the block sums become their exclusive prefix sums, the
+// word after them the total.
+__global__ void __launch_bounds__(kScanBlock)
+scan_blocks_kernel(int64_t nb, const ScanPair S) {
+    int64_t *block_sums = S.ws[blockIdx.y];
     const int64_t chunk = (nb + blockDim.x - 1) / blockDim.x;
-    const int64_t b0 = threadIdx.x * chunk, b1 = min(nb, b0 + chunk);
-    int64_t acc = 0;
-    for (int64_t b = b0; b < b1; b++) acc += block_sums[b];
-    s[threadIdx.x] = acc;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        int64_t run = 0;
-        for (int t = 0; t < (int)blockDim.x; t++) { const int64_t c = s[t]; s[t] = run; run += c; }
-        *total = run;
-    }
-    __syncthreads();
-    acc = s[threadIdx.x];
+    const int64_t b0 = min(nb, threadIdx.x * chunk), b1 = min(nb, b0 + chunk);
+    int64_t mine = 0;
+    for (int64_t b = b0; b < b1; b++) mine += block_sums[b];
+    const int64_t s = block_scan(mine);
+    if (threadIdx.x == blockDim.x - 1) block_sums[nb] = s;
+    int64_t acc = s - mine;
     for (int64_t b = b0; b < b1; b++) { const int64_t c = block_sums[b]; block_sums[b] = acc; acc += c; }
 }
 
-__global__ void scan_add_kernel(int64_t n, int32_t *__restrict__ out, const int64_t *__restrict__ block_sums,
-                                const int64_t *__restrict__ total) {
+__global__ void scan_add_kernel(int64_t n, int64_t nb, const ScanPair S) {
     const int64_t i = (int64_t)blockIdx.x * kScanBlock + threadIdx.x;
-    if (i < n) out[i] = (int32_t)(out[i] + block_sums[blockIdx.x]);
-    if (i == n) out[n] = (int32_t)*total;
+    int32_t *out = S.out[blockIdx.y];
+    if (i < n) out[i] = (int32_t)(out[i] + S.ws[blockIdx.y][blockIdx.x]);
+    if (i == n) out[n] = (int32_t)S.ws[blockIdx.y][nb];
+}
+
+// The same in one launch for up to kScanSmall entries, kScanEach a thread.
+constexpr int kScanEach = 8;
+constexpr int64_t kScanSmall = (int64_t)kScanEach * kScanBlock - 1;
+
+__global__ void __launch_bounds__(kScanBlock)
+scan_small_kernel(int n, const ScanPair S) {
+    const int32_t *in = S.in[blockIdx.y];
+    int32_t *out = S.out[blockIdx.y];
+    const int i0 = threadIdx.x * kScanEach;
+    int64_t v[kScanEach], mine = 0;
+#pragma unroll
+    for (int k = 0; k < kScanEach; k++) {
+        v[k] = i0 + k < n ? in[i0 + k] : 0;
+        mine += v[k];
+    }
+    int64_t acc = block_scan(mine) - mine;
+#pragma unroll
+    for (int k = 0; k < kScanEach; k++) {
+        if (i0 + k <= n) out[i0 + k] = (int32_t)acc;
+        acc += v[k];
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -784,7 +858,10 @@ row_walk_kernel(int64_t ndof, const int32_t *__restrict__ inc_ptr, const int32_t
         for (int o = 16; o > 0; o >>= 1) maxwalk = max(maxwalk, __shfl_xor_sync(0xffffffffu, maxwalk, o));
         if (maxwalk == 0) continue;   // warp-uniform
 
-        for (int t = gl; t < HS; t += G) key[t] = -1;
+        // the part of the table rows of that many incidences need (half of it
+        // holds a P2 edge's or a P3 face's row, and is cleared in half the time)
+        const int hs = maxwalk * N <= HS / 2 - HS / 8 ? HS / 2 : HS;
+        for (int t = gl; t < hs; t += G) key[t] = -1;
         __syncwarp();
         int L = 0;
         bool overflow = false;
@@ -831,22 +908,22 @@ row_walk_kernel(int64_t ndof, const int32_t *__restrict__ inc_ptr, const int32_t
             const bool nz = f0.ok != 0 && v != 0.0;
             int pos = -1;
             if (nz) {
-                unsigned h = hash32(col) & (HS - 1);
-                for (int probe = 0; probe < HS; probe++) {
+                unsigned h = hash32(col) & (hs - 1);
+                for (int probe = 0; probe < hs; probe++) {
                     const int32_t k = key[h];
                     if (k == col) { pos = hpos[h]; break; }
                     if (k == -1) break;
-                    h = (h + 1) & (HS - 1);
+                    h = (h + 1) & (hs - 1);
                 }
             }
             const unsigned newm = __ballot_sync(0xffffffffu, nz && pos < 0) & gmask;
             if (nz && pos < 0) {
                 pos = L + __popc(newm & lt_mask);
                 if (pos < MAXROW) {
-                    unsigned h = hash32(col) & (HS - 1);
-                    for (int probe = 0; probe < HS; probe++) {
+                    unsigned h = hash32(col) & (hs - 1);
+                    for (int probe = 0; probe < hs; probe++) {
                         if (atomicCAS(&key[h], -1, col) == -1) { hpos[h] = (int16_t)pos; break; }
-                        h = (h + 1) & (HS - 1);
+                        h = (h + 1) & (hs - 1);
                     }
                     scol[pos] = col;
                     sval[pos] = v;
@@ -928,11 +1005,11 @@ row_walk_kernel(int64_t ndof, const int32_t *__restrict__ inc_ptr, const int32_t
         // element right-hand sides of this row, loaded by the lanes in parallel
         // and added by the group's first lane in element order (zeros skipped)
         double r = 0.0;
-        for (int t = 0; t < G; t++) {
+        for (int t = 0; t < min(G, maxwalk); t++) {
             const double ba = __shfl_sync(0xffffffffu, reA, t, G);
             if (gl == 0 && t < nwalk && ba != 0.0) r = rn_add(r, ba);
         }
-        for (int t = 0; t < G; t++) {
+        for (int t = 0; t < min(G, maxwalk - G); t++) {
             const double bb = __shfl_sync(0xffffffffu, reB, t, G);
             if (gl == 0 && G + t < nwalk && bb != 0.0) r = rn_add(r, bb);
         }
@@ -1081,7 +1158,7 @@ value_walk_kernel(int64_t ndof, const int32_t *__restrict__ inc_ptr, const int32
                 __syncwarp();
             }
             // the chunk's element RHS entries, zeros skipped
-            for (int t = 0; t < G; t++) {
+            for (int t = 0; t < maxj; t++) {
                 const double bt = __shfl_sync(0xffffffffu, reb, t, G);
                 if (gl == 0 && c0 + t < nwalk && bt != 0.0) r = rn_add(r, bt);
             }
@@ -1304,25 +1381,24 @@ template <int P>
 static void elem_launch(const ElemArgs &A, cudaStream_t s) {
     constexpr int W = ElemDims<P>::WARPS;
     if (!A.geometry_given)
-        geometry_kernel<<<grid_for(A.nelem, 128, 148 * 64), 128, 0, s>>>(A.nelem, A.nvert, A.verts, A.elems,
+        geometry_kernel<<<grid_for(A.nelem, kGeoThreads, 148 * 64), kGeoThreads, 0, s>>>(A.nelem, A.nvert, A.verts, A.elems,
                                                                         A.geo, A.status);
     ElemWeights Wt{};
     for (int q = 0; q < ElemDims<P>::QK; q++) Wt.wk[q] = A.wk_host[q];
-    for (int q = 0; q < ElemDims<P>::QR; q++) Wt.wr[q] = A.wr_host[q];
     if constexpr (P == 1) {   // a lane per basis function
         constexpr int EPB = 4 * (32 / ElemDims<P>::N);   // elements per block
         const int blocks = grid_for(A.nelem, EPB, 148 * 64);
         element_lanes_kernel<P><<<blocks, 128, 0, s>>>(A.nelem, A.ndof, A.geo, A.e2l, A.kappa, A.mass, A.f, Wt,
-                                                       A.gk, A.br, A.brt, A.Ke, A.Re, A.status);
+                                                       A.gk, A.mt, A.bw, A.brt, A.Ke, A.Re, A.status);
     } else if constexpr (P == 2) {   // a lane per two basis functions
         constexpr int EPB = 4 * (32 / (ElemDims<P>::N / 2));
         const int blocks = grid_for(A.nelem, EPB, 148 * 64);
         element_cols2_kernel<P><<<blocks, 128, 0, s>>>(A.nelem, A.ndof, A.geo, A.e2l, A.kappa, A.mass, A.f, Wt,
-                                                       A.gk, A.br, A.brt, A.Ke, A.Re, A.status);
+                                                       A.gk, A.mt, A.bw, A.brt, A.Ke, A.Re, A.status);
     } else {          // P3: a warp per element
         const int blocks = grid_for(A.nelem, W, 148 * 64);
         element_kernel<P><<<blocks, W * 32, 0, s>>>(A.nelem, A.ndof, A.geo, A.e2l, A.kappa, A.mass, A.f, Wt, A.gk,
-                                                    A.br, A.brt, A.Ke, A.Re, A.status);
+                                                    A.mt, A.bw, A.brt, A.Ke, A.Re, A.status);
     }
 }
 
@@ -1348,20 +1424,33 @@ cudaError_t launch_incidence(int N, int64_t nelem, int64_t ndof, const int32_t *
     cudaError_t err = launch_scan(ndof, cnt, inc_ptr, scan_ws, s);
     if (err != cudaSuccess) return err;
     inc_fill_kernel<<<bl, 256, 0, s>>>(nkeys, ndof, e2l, inc_ptr, cursor, inc);
-    inc_sort_kernel<<<grid_for(ndof, 128, 148 * 16), 128, 0, s>>>(ndof, inc_ptr, inc);
+    inc_sort_kernel<<<grid_for(ndof * 8, 128, 148 * 16), 128, 0, s>>>(ndof, inc_ptr, inc);
     return cudaGetLastError();
 }
 
-int64_t scan_workspace_elems(int64_t n) { return ceil_div(n + 1, kScanBlock) + 2; }
+int64_t scan_workspace_elems(int64_t n) { return 2 * (ceil_div(n + 1, kScanBlock) + 1); }
+
+int scan_launches(int64_t n) { return n <= kScanSmall ? 1 : 3; }
+
+static cudaError_t scan_arrays(int64_t n, int arrays, const ScanPair &S, cudaStream_t s) {
+    if (n <= kScanSmall) {   // one launch of 3 us instead of three of 10
+        scan_small_kernel<<<dim3(1, arrays), kScanBlock, 0, s>>>((int)n, S);
+        return cudaGetLastError();
+    }
+    const int64_t nb = ceil_div(n + 1, kScanBlock);
+    scan_local_kernel<<<dim3((unsigned)nb, arrays), kScanBlock, 0, s>>>(n, S);
+    scan_blocks_kernel<<<dim3(1, arrays), kScanBlock, 0, s>>>(nb, S);
+    scan_add_kernel<<<dim3((unsigned)nb, arrays), kScanBlock, 0, s>>>(n, nb, S);
+    return cudaGetLastError();
+}
 
 cudaError_t launch_scan(int64_t n, const int32_t *in, int32_t *out, int64_t *ws, cudaStream_t s) {
-    // ws: block sums (nb) + total; out has n + 1 entries
-    const int64_t nb = ceil_div(n + 1, kScanBlock);
-    int64_t *total = ws + nb;
-    scan_local_kernel<<<(unsigned)nb, kScanBlock, 0, s>>>(n, in, out, ws);
-    scan_blocks_kernel<<<1, 1024, 0, s>>>(nb, ws, total);
-    scan_add_kernel<<<(unsigned)nb, kScanBlock, 0, s>>>(n, out, ws, total);
-    return cudaGetLastError();
+    return scan_arrays(n, 1, ScanPair{{in, nullptr}, {out, nullptr}, {ws, nullptr}}, s);
+}
+
+cudaError_t launch_scan2(int64_t n, const int32_t *in0, int32_t *out0, const int32_t *in1, int32_t *out1, int64_t *ws,
+                         cudaStream_t s) {
+    return scan_arrays(n, 2, ScanPair{{in0, in1}, {out0, out1}, {ws, ws + ceil_div(n + 1, kScanBlock) + 1}}, s);
 }
 
 template <int N>

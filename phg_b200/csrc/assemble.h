@@ -17,10 +17,12 @@ struct ElemArgs {
     const double *kappa, *f;                 // may be null
     double mass;                             // mass coefficient c (0: stiffness only)
     // element tables (device): gk = d phi_k / d lambda_c at stiffness point q
-    // as gk[(c * QK + q) * N + k]; br = phi_k at rhs point q as br[q * N + k],
-    // brt the same transposed (brt[k * QR + q])
-    const double *gk, *br, *brt;
-    const double *wk_host, *wr_host;         // quadrature weights (host; passed by value)
+    // as gk[(c * QK + q) * N + k]; brt = phi_k at rhs point q as brt[k * QR + q];
+    // bw = phi_k times the point's weight as bw[q * N + k]; mt = the sum of
+    // phi_a phi_b times the weights over the points (the mass matrix without
+    // the volume) as mt[a * N + b]
+    const double *gk, *brt, *bw, *mt;
+    const double *wk_host;                   // stiffness weights (host; passed by value)
     double *geo;                             // nelem * geometry_doubles: J (16), volume per element
     bool geometry_given;                     // geo holds the caller's geometry (else computed here)
     double *Ke, *Re;
@@ -59,6 +61,11 @@ cudaError_t launch_incidence(int N, int64_t nelem, int64_t ndof, const int32_t *
 int64_t scan_workspace_elems(int64_t n);
 // out[0..n] = exclusive prefix sums of in[0..n-1], out[n] = total (int32).
 cudaError_t launch_scan(int64_t n, const int32_t *in, int32_t *out, int64_t *ws, cudaStream_t s);
+// Kernels a scan of n entries launches.
+int scan_launches(int64_t n);
+// The same for two arrays at once.
+cudaError_t launch_scan2(int64_t n, const int32_t *in0, int32_t *out0, const int32_t *in1, int32_t *out1, int64_t *ws,
+                         cudaStream_t s);
 // One pass over the rows into the scratch regions (counts, RHS, diagonal),
 // then, after the counts are scanned into ptr/bptr, the copy into the CSR.
 cudaError_t launch_row_walk(int p, const WalkArgs &a, cudaStream_t s);

@@ -178,8 +178,8 @@ struct phgGpuSystem_ {
 
     // element tables
     int tab_order = 0;
-    DevBuf<double> gk, br, brt;            // basis derivatives / values at the points (device)
-    std::vector<double> wk, wr;            // quadrature weights (passed to the kernel by value)
+    DevBuf<double> gk, brt, bw, mt;        // basis derivatives / values at the points, mass sums (device)
+    std::vector<double> wk;                // stiffness weights (passed to the kernel by value)
 
     // assembly buffers
     DevBuf<double> Ke, Re, kappa, f, g, geo;
@@ -221,7 +221,7 @@ struct phgGpuSystem_ {
     DevBuf<int64_t> tmp64;
     PcgState *h_st = nullptr;
     double *h_sums = nullptr;
-    int *h_status = nullptr;
+    int *h_status = nullptr;               // the status word, then the entry counts of a build
     DevBuf<int> status;
     cudaGraphExec_t graph = nullptr;
     struct GraphKey {
@@ -363,23 +363,40 @@ int upload_tables(phgGpuSystem *s, int p) {
     const ElementTables t = make_tables(p);
     if ((int)t.wk.size() > kElemMaxQK || (int)t.wr.size() > kElemMaxQR)
         return fail(PHG_GPU_ERR_LIMIT, "quadrature rule larger than the element kernel's");
-    // the kernel reads gk component-major with the basis index fastest, and
-    // br both point-major (the RHS sums) and basis-major (f_h at the points)
+    // the kernel reads gk component-major with the basis index fastest, the
+    // basis values basis-major (f_h at the points) and times the weights
+    // point-major (the RHS sums), and the mass sums, each product and sum
+    // rounded as the reference rounds it
     const int N = t.N, QK = t.nq_k, QR = t.nq_r;
     std::vector<double> gkc(t.gk.size()), brt(t.br.size());
     for (int q = 0; q < QK; q++)
         for (int k = 0; k < N; k++)
             for (int c = 0; c < 4; c++) gkc[((size_t)c * QK + q) * N + k] = t.gk[((size_t)q * N + k) * 4 + c];
+    std::vector<double> bw(t.br.size()), mt((size_t)N * N);
     for (int q = 0; q < QR; q++)
-        for (int k = 0; k < N; k++) brt[(size_t)k * QR + q] = t.br[(size_t)q * N + k];
+        for (int k = 0; k < N; k++) {
+            brt[(size_t)k * QR + q] = t.br[(size_t)q * N + k];
+            bw[(size_t)q * N + k] = t.br[(size_t)q * N + k] * t.wr[q];
+        }
+    for (int a = 0; a < N; a++)
+        for (int b = 0; b < N; b++) {
+            double dm = 0.0;
+            for (int q = 0; q < QR; q++) {
+                const double d0 = t.br[(size_t)q * N + b] * t.br[(size_t)q * N + a];
+                const double d1 = d0 * t.wr[q];
+                dm = dm + d1;
+            }
+            mt[(size_t)a * N + b] = dm;
+        }
     CHECK_RC(s->gk.ensure(gkc.size()));
-    CHECK_RC(s->br.ensure(t.br.size()));
+    CHECK_RC(s->bw.ensure(bw.size()));
+    CHECK_RC(s->mt.ensure(mt.size()));
     CHECK_RC(s->brt.ensure(brt.size()));
     CK(cudaMemcpy(s->gk.p, gkc.data(), gkc.size() * sizeof(double), cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(s->br.p, t.br.data(), t.br.size() * sizeof(double), cudaMemcpyHostToDevice));
+    CK(cudaMemcpy(s->bw.p, bw.data(), bw.size() * sizeof(double), cudaMemcpyHostToDevice));
+    CK(cudaMemcpy(s->mt.p, mt.data(), mt.size() * sizeof(double), cudaMemcpyHostToDevice));
     CK(cudaMemcpy(s->brt.p, brt.data(), brt.size() * sizeof(double), cudaMemcpyHostToDevice));
     s->wk = t.wk;
-    s->wr = t.wr;
     s->tab_order = p;
     return PHG_GPU_OK;
 }
@@ -461,7 +478,7 @@ int ensure_sell(phgGpuSystem *s) {
     CHECK_RC(s->sell_vals32.ensure((size_t)total));
     CK(launch_sell_fill(n, s->rp.p, s->ci.p, s->va.p, s->sell_perm.p, s->sell_len.p, s->sell_sptr.p,
                         s->sell_cols.p, s->sell_vals.p, s->sell_vals32.p, s->stream));
-    s->launches += 4;
+    s->launches += 1 + scan_launches(nsl);
     s->sell_total = total;
     s->sell_valid = true;
     return PHG_GPU_OK;
@@ -521,7 +538,7 @@ int ensure_sell2(phgGpuSystem *s) {
     CHECK_RC(s->sell2_len.ensure((size_t)nsl * 32));
     CK(launch_sell2_fill(S, s->rp.p, s->ci.p, s->va.p, s->sell2_order.p, s->sell2_sptr.p, s->sell2_perm.p,
                          s->sell2_len.p, s->sell2_cols.p, s->sell2_vals.p, s->stream));
-    s->launches += 3;
+    s->launches += 2 + scan_launches(nsl);
     s->sell2_total = total;
     s->sell2_valid = true;
     return PHG_GPU_OK;
@@ -574,7 +591,7 @@ int ensure_q16(phgGpuSystem *s) {
                        s->q16_nofit.p, s->stream));
     CK(cudaMemcpyAsync(s->h_nofit, s->q16_nofit.p, sizeof(int), cudaMemcpyDeviceToHost, s->stream));
     CK(cudaStreamSynchronize(s->stream));
-    s->launches += 3;
+    s->launches += 2 + scan_launches(nsl);
     s->q16_total = total;
     s->q16_valid = true;
     s->q16_fits = *s->h_nofit == 0;
@@ -796,7 +813,7 @@ int phgGpuCreate(int device, void *stream, phgGpuSystem **out) {
     if (rc == PHG_GPU_OK) {
         cudaError_t e1 = cudaMallocHost((void **)&s->h_st, sizeof(PcgState));
         cudaError_t e2 = cudaMallocHost((void **)&s->h_sums, 4 * sizeof(double));
-        cudaError_t e3 = cudaMallocHost((void **)&s->h_status, sizeof(int));
+        cudaError_t e3 = cudaMallocHost((void **)&s->h_status, 3 * sizeof(int));
         if (e1 != cudaSuccess || e2 != cudaSuccess || e3 != cudaSuccess)
             rc = fail(PHG_GPU_ERR_CUDA, "cudaMallocHost failed");
     }
@@ -850,7 +867,7 @@ int phgGpuDestroy(phgGpuSystem *s) {
     for (auto *b : bf) b->release();
     s->bint.release();
     s->btick.release();
-    DevBuf<double> *dbufs[] = {&s->verts, &s->gk, &s->br, &s->brt, &s->Ke, &s->Re, &s->kappa, &s->f,
+    DevBuf<double> *dbufs[] = {&s->verts, &s->gk, &s->brt, &s->bw, &s->mt, &s->Ke, &s->Re, &s->kappa, &s->f,
                                &s->g, &s->geo, &s->va, &s->bva, &s->rhs, &s->diag, &s->x, &s->r, &s->p, &s->Ap,
                                &s->partials, &s->hist, &s->sums};
     for (auto *b : dbufs) b->release();
@@ -960,7 +977,7 @@ int phgGpuSetDofMap(phgGpuSystem *s, int order, int64_t ndof, const int32_t *e2l
     CHECK_RC(upload_tables(s, order));
     CK(launch_incidence(N, s->nelem, ndof, s->e2l.p, s->cnt.p, s->inc_ptr.p, s->cursor.p, s->inc.p,
                         s->scan_ws.p, s->status.p, s->stream));
-    s->launches += 6;
+    s->launches += 3 + scan_launches(ndof);
     s->order = order;
     s->N = N;
     s->ndof = ndof;
@@ -986,7 +1003,7 @@ static int element_pass(phgGpuSystem *s, const double *kappa, double mass, const
     ea.nelem = s->nelem; ea.nvert = s->nvert; ea.ndof = ndof;
     ea.verts = s->verts.p; ea.elems = s->elems.p; ea.e2l = s->e2l.p;
     ea.kappa = dk; ea.f = df; ea.mass = mass;
-    ea.gk = s->gk.p; ea.br = s->br.p; ea.brt = s->brt.p; ea.wk_host = s->wk.data(); ea.wr_host = s->wr.data();
+    ea.gk = s->gk.p; ea.brt = s->brt.p; ea.bw = s->bw.p; ea.mt = s->mt.p; ea.wk_host = s->wk.data();
     ea.Ke = s->Ke.p; ea.Re = s->Re.p; ea.geo = s->geo.p; ea.status = s->status.p;
     // the geometry is computed once per mesh (a build that succeeded has
     // checked its vertex indices and coordinates)
@@ -1061,11 +1078,10 @@ static int build_system(phgGpuSystem *s, const double *kappa, double mass, const
         wa.dpos = nullptr;
     }
     CK(launch_row_walk(s->order, wa, s->stream));
-    s->launches += 8;   // walk (two passes) + two scans
-    CK(launch_scan(ndof, s->cnt_keep.p, s->rp.p, s->scan_ws.p, s->stream));
-    int32_t tot[2];
+    s->launches += 2 + scan_launches(ndof);   // walk (two passes) + scans
+    CK(launch_scan2(ndof, s->cnt_keep.p, s->rp.p, s->cnt_bdry.p, s->brp.p, s->scan_ws.p, s->stream));
+    int32_t *tot = s->h_status + 1;   // pinned: the copies return at once, the check below waits for them
     CK(cudaMemcpyAsync(&tot[0], s->rp.p + ndof, sizeof(int32_t), cudaMemcpyDeviceToHost, s->stream));
-    CK(launch_scan(ndof, s->cnt_bdry.p, s->brp.p, s->scan_ws.p, s->stream));
     CK(cudaMemcpyAsync(&tot[1], s->brp.p + ndof, sizeof(int32_t), cudaMemcpyDeviceToHost, s->stream));
     CHECK_RC(check_status(s, "phgGpuBuildLinearSystem (rows)"));
     s->geometry_valid = true;
@@ -1220,7 +1236,7 @@ int phgGpuAssembleRows(phgGpuSystem *s, int64_t n, int64_t nrec, const int32_t *
     CK(cudaMemcpyAsync(&tot, s->rp.p + n, sizeof(int32_t), cudaMemcpyDeviceToHost, s->stream));
     CK(cudaMemcpyAsync(s->h_status, s->status.p, sizeof(int), cudaMemcpyDeviceToHost, s->stream));
     CK(cudaStreamSynchronize(s->stream));
-    s->launches += 12;
+    s->launches += 6 + 3 * scan_launches(n);
     const int st = *s->h_status;
     if (st != PHGB_DEV_OK) {
         *s->h_status = 0;
