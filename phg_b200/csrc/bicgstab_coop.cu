@@ -33,7 +33,7 @@ bicg_coop_kernel(const BicgRun R) {
     __shared__ CoopShared sh;
     __shared__ BicgScalars S;
     __shared__ int next_unit;
-    CoopGrid G(R.exchange, &sh);
+    CoopGrid<> G(R.exchange, &sh);
     const int t = threadIdx.x;
     const unsigned n = (unsigned)R.A.n;
     const int m = coop_places(n);

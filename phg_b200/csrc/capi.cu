@@ -1456,11 +1456,17 @@ int phgGpuSolverPCGMixed(phgGpuSystem *s, double rtol, double btol, double atol,
                             s->sell_vals.p, s->sell_vals32.p, s->s32.p, s->partials.p};
         memcpy(key.extra, e, sizeof(e));
     }
-    if (s->graph_mixed == nullptr || !(s->gkey_mixed == key)) {
+    // the q16 layout's iterations run as one cooperative kernel, the other
+    // layouts' as a graph
+    bool one_kernel = q16 && !s->plain_graphs;
+    if (one_kernel) CHECK_RC(s->coop_xch.ensure((size_t)coop_exchange_doubles()));
+    auto mixed_graph = [&]() -> int {
+        if (s->graph_mixed != nullptr && s->gkey_mixed == key) return PHG_GPU_OK;
         if (s->graph_mixed != nullptr) { cudaGraphExecDestroy(s->graph_mixed); s->graph_mixed = nullptr; }
         CK(build_gear_graph(B, L, kGraphChunk, s->plain_graphs, s->stream, &s->graph_mixed, nullptr));
         s->gkey_mixed = key;
-    }
+        return PHG_GPU_OK;
+    };
     // the explicit FP64 residual b - A x is checked at the end; a recurrence
     // that drifted above the tolerance restarts from it (at most twice)
     for (int restart = 0; restart < 3; restart++) {
@@ -1498,7 +1504,14 @@ int phgGpuSolverPCGMixed(phgGpuSystem *s, double rtol, double btol, double atol,
         CK(cudaMemcpyAsync(s->gst.p, s->h_gst_mixed, sizeof(GearState), cudaMemcpyHostToDevice, s->stream));
         int plain_passes = 0;
         bool plain_limit = false;
-        if (!g.done && !s->plain_graphs) CK(cudaGraphLaunch(s->graph_mixed, s->stream));
+        if (!g.done && one_kernel) {
+            CK(cudaMemsetAsync(s->coop_xch.p, 0, sizeof(double) * coop_exchange_doubles(), s->stream));
+            const cudaError_t e = launch_gear_coop(B, Q, s->unroll32, s->coop_xch.p, s->stream);
+            if (e == cudaErrorNotSupported) one_kernel = false;
+            else CK(e);
+        }
+        if (!g.done && !one_kernel) CHECK_RC(mixed_graph());
+        if (!g.done && !one_kernel && !s->plain_graphs) CK(cudaGraphLaunch(s->graph_mixed, s->stream));
         if (!g.done && s->plain_graphs) {
             for (;;) {
                 if (plain_passes >= g.max_passes) { plain_limit = true; break; }
@@ -1515,6 +1528,7 @@ int phgGpuSolverPCGMixed(phgGpuSystem *s, double rtol, double btol, double atol,
         GearState &hg = *s->h_gst_mixed;
         if (plain_limit) hg.status = GEAR_PASS_LIMIT;
         if (s->plain_graphs) s->launches += 4 * (int64_t)kGraphChunk * plain_passes + 1;
+        else if (one_kernel) s->launches += 2;
         else s->launches += 2 * (int64_t)hg.nits + 2 * (int64_t)hg.nupdates + hg.passes + 1;
         nits_total += hg.nits;
         nupd += hg.nupdates;

@@ -95,7 +95,7 @@ gmres_coop_kernel(const GmresRun R) {
     __shared__ CoopShared sh;
     __shared__ GmresScalars S;
     __shared__ int next_unit;
-    CoopGrid G(R.exchange, &sh);
+    CoopGrid<> G(R.exchange, &sh);
     const int t = threadIdx.x;
     const unsigned n = (unsigned)R.A.n;
     const int m = coop_places(n);

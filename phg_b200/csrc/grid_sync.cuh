@@ -27,12 +27,13 @@ namespace phgb {
 
 constexpr int kCoopThreads = 1024;   // one block an SM: 64 registers a thread
 constexpr int kCoopWarps = kCoopThreads / 32;
-constexpr int kCoopMaxBlocks = 160;  // five partials a lane of the adding warp
+constexpr int kCoopMaxBlocks = 160;  // of the solvers with a block an SM
+constexpr int kCoopMostBlocks = 320; // of any grid
 constexpr int kCoopSums = 3;         // sums exchanged at once, at most
 // Doubles of exchange memory, zero before the launch: two buffers of partials
 // (a block may be writing the next sum while another still reads the last),
 // then two 32-bit words, the arrivals and the give-up flag.
-constexpr int kCoopDoubles = 2 * kCoopSums * kCoopMaxBlocks + 1;
+constexpr int kCoopDoubles = 2 * kCoopSums * kCoopMostBlocks + 1;
 // Polls before a wait gives up (each is an L2 round trip, about half a
 // microsecond: some ten seconds).
 constexpr int kCoopPolls = 1 << 24;
@@ -42,6 +43,8 @@ struct CoopShared {
     int failed;
 };
 
+// MAXB: blocks of the grid at most (MAXB / 32 partials a lane of the adding warp).
+template <int MAXB = kCoopMaxBlocks>
 struct CoopGrid {
     double *mem;        // kCoopDoubles
     CoopShared *sh;
@@ -80,26 +83,26 @@ struct CoopGrid {
             for (int k = 0; k < K; k++) t[k] = warp_sum(sh->part[k][lane]);
             int ok = 1;
             if (gridDim.x > 1) {
-                double *P = mem + (epoch & 1u) * (kCoopSums * kCoopMaxBlocks);   // [sum][block]
+                double *P = mem + (epoch & 1u) * (kCoopSums * MAXB);   // [sum][block]
                 if (lane == 0) {
 #pragma unroll
-                    for (int k = 0; k < K; k++) P[k * kCoopMaxBlocks + blockIdx.x] = t[k];
+                    for (int k = 0; k < K; k++) P[k * MAXB + blockIdx.x] = t[k];
                     ok = arrive_wait() ? 1 : 0;
                 }
                 __syncwarp();   // the lanes' loads below come after lane 0's acquire
-                double a[K][kCoopMaxBlocks / 32];
+                double a[K][MAXB / 32];
 #pragma unroll
                 for (int k = 0; k < K; k++)
 #pragma unroll
-                    for (int j = 0; j < kCoopMaxBlocks / 32; j++) {
+                    for (int j = 0; j < MAXB / 32; j++) {
                         const unsigned b = lane + 32 * j;
-                        a[k][j] = b < gridDim.x ? fetch(&P[k * kCoopMaxBlocks + b]) : 0.0;
+                        a[k][j] = b < gridDim.x ? fetch(&P[k * MAXB + b]) : 0.0;
                     }
 #pragma unroll
                 for (int k = 0; k < K; k++) {
                     t[k] = a[k][0];
 #pragma unroll
-                    for (int j = 1; j < kCoopMaxBlocks / 32; j++) t[k] += a[k][j];
+                    for (int j = 1; j < MAXB / 32; j++) t[k] += a[k][j];
                     t[k] = warp_sum(t[k]);
                 }
             }
@@ -122,7 +125,7 @@ private:
     // One thread of the block: arrive and wait for every block.  False when
     // the wait gave up here or elsewhere.
     __device__ __forceinline__ bool arrive_wait() const {
-        unsigned *bar = reinterpret_cast<unsigned *>(mem + 2 * kCoopSums * kCoopMaxBlocks);
+        unsigned *bar = reinterpret_cast<unsigned *>(mem + kCoopDoubles - 1);
         const unsigned target = epoch * gridDim.x;
         asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
         for (int i = 0; i < kCoopPolls; i++) {

@@ -29,6 +29,7 @@
 // The iterations run in a conditional WHILE loop of `chunk` iterations per
 // pass, so a solve is one graph launch and the host waits once.
 #include "common.cuh"
+#include "grid_sync.cuh"
 #include "mixed.h"
 #include "reduce.cuh"
 #include "rows.cuh"
@@ -89,6 +90,25 @@ __device__ __forceinline__ bool gear_check(GearState *st, double rr) {
     const bool conv = !(res > st->tol) || st->nits >= st->maxit;
     st->final_check = conv ? 1 : 0;
     return conv || res < st->delta * st->maxr;
+}
+
+// After a reliable update: v = (||rtrue||^2, r.u, r.r) of the restarted
+// recurrence.
+__device__ __forceinline__ void gear_updated(GearState *st, const double *v) {
+    const double res = sqrt(v[0]);
+    st->residual = res;
+    st->maxr = res;
+    st->gamma_cur = v[1];
+    st->rr_cur = v[2];
+    st->y_reset = 1;
+    st->nupdates += 1;
+    st->final_check = 0;
+    if (!isfinite(res)) {
+        st->done = 1;
+        st->status = PCG_NONFINITE;
+    } else if (!(res > st->tol) || st->nits >= st->maxit) {
+        st->done = 1;   // the FP64 residual meets the tolerance, or maxit
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -163,22 +183,7 @@ gear_reliable_kernel(const L64 lay, const GearBuffers B) {
             v[2] += (double)rf * (double)rf;
         }
     }
-    if (grid_sum3(v, B.partials, st->ticket)) {
-        const double res = sqrt(v[0]);
-        st->residual = res;
-        st->maxr = res;
-        st->gamma_cur = v[1];
-        st->rr_cur = v[2];
-        st->y_reset = 1;
-        st->nupdates += 1;
-        st->final_check = 0;
-        if (!isfinite(res)) {
-            st->done = 1;
-            st->status = PCG_NONFINITE;
-        } else if (!(res > st->tol) || st->nits >= st->maxit) {
-            st->done = 1;   // the FP64 residual meets the tolerance, or maxit
-        }
-    }
+    if (grid_sum3(v, B.partials, st->ticket)) gear_updated(st, v);
 }
 
 // K2: the vector update, V rows a thread and step (16-byte vectors: 2.5% to
@@ -273,6 +278,171 @@ gear_update_kernel(const GearBuffers B, cudaGraphConditionalHandle hif) {
         st->ru_due = due ? 1 : 0;
         if constexpr (COND) cudaGraphSetConditional(hif, due ? 1u : 0u);
     }
+}
+
+// The iterations on the q16 layout as one cooperative kernel: the phases of K1,
+// K2, R0 and R1 between grid barriers that carry their sums, for matrices
+// whose vectors do not fit the SMs' shared memory (mixed_coop.cu).  The vectors
+// go through L2; two blocks of 1024 threads an SM keep as many warps at the
+// product as its own launch would (with one block an SM it waits for memory).
+// As launches, an iteration spends a third of its time outside the product and
+// the update's bytes: launches, ramps, two ticket sums and a conditional node.
+// Per iteration, us: P2 64^3 (2.1 million rows, 57 million entries) 104 (107 as
+// launches), P2 705k rows 48.9 (51.3), P1 1.03 million rows 35.8 (41.1); the
+// product's blocks finish some 10 us apart at 64^3.  (One block an SM with 64
+// registers and twice the unrolling: 145 us at P2 64^3.)
+constexpr int kGearCoopThreads = 1024;
+
+// One step's FP32 row sum (Q16Rows32::sum, with plain loads of x: other blocks
+// wrote it before the last barrier).
+template <int U>
+__device__ __forceinline__ float q16_sum_rw(const Q16View &Q, int s, int lane, int pos, const float *x) {
+    const int l = Q.len[pos];
+    const int sp = Q.split[pos];
+    const int32_t b0 = Q.base0[pos], b1 = Q.base1[pos];
+    const int wq = (__shfl_sync(0xffffffffu, l, 0) + 3) >> 2;
+    const uint2 *cp = reinterpret_cast<const uint2 *>(Q.cols + Q.sptr[s]) + lane;
+    const float4 *vp = reinterpret_cast<const float4 *>(Q.vals32 + Q.sptr[s]) + lane;
+    float acc = 0.0f;
+    for (int jq = 0; jq < wq; jq += U) {
+        uint2 c[U];
+        float4 v[U];
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const bool ok = 4 * (jq + u) < l;
+            c[u] = ok ? __ldcs(cp + 32 * (jq + u)) : make_uint2(0u, 0u);
+            v[u] = ok ? __ldcs(vp + 32 * (jq + u)) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        }
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const int j = 4 * (jq + u);
+            if (j < l) acc = fma_free(acc, v[u].x, x[q16_col(j, sp, b0, b1, c[u].x & 0xffffu)]);
+            if (j + 1 < l) acc = fma_free(acc, v[u].y, x[q16_col(j + 1, sp, b0, b1, c[u].x >> 16)]);
+            if (j + 2 < l) acc = fma_free(acc, v[u].z, x[q16_col(j + 2, sp, b0, b1, c[u].y & 0xffffu)]);
+            if (j + 3 < l) acc = fma_free(acc, v[u].w, x[q16_col(j + 3, sp, b0, b1, c[u].y >> 16)]);
+        }
+    }
+    return acc;
+}
+
+template <int U>
+__global__ void __launch_bounds__(kGearCoopThreads, 2)
+gear_coop_kernel(const Q16View Q, const GearBuffers B, double *exchange) {
+    __shared__ CoopShared sh;
+    __shared__ GearState S;
+    CoopGrid<kCoopMostBlocks> G(exchange, &sh);
+    const int lane = threadIdx.x & 31;
+    const int tid = blockIdx.x * kGearCoopThreads + threadIdx.x, nthreads = gridDim.x * kGearCoopThreads;
+    const int warp = tid >> 5, nwarps = nthreads >> 5;
+    const int nsl = (int)Q.nslices, n = (int)B.n;   // n < 2^31 - the grid's threads
+    for (int i = threadIdx.x; i < (int)(sizeof(GearState) / 4); i += kGearCoopThreads)
+        reinterpret_cast<unsigned *>(&S)[i] = reinterpret_cast<const unsigned *>(B.st)[i];
+    __syncthreads();
+    bool ok = true;
+    double d[1], v[2], v3[3];
+    while (ok && !S.done) {
+        // K1
+        d[0] = 0.0;
+        for (int s = warp; s < nsl; s += nwarps) {
+            const int pos = s * 32 + lane;
+            const int32_t row = Q.perm[pos];
+            const float uf = row >= 0 ? B.u[row] : 0.0f;
+            const float acc = q16_sum_rw<U>(Q, s, lane, pos, B.u);
+            if (row >= 0) {
+                B.w[row] = acc;
+                d[0] += (double)acc * (double)uf;
+            }
+        }
+        ok = G.sum(d, [&](const double *t) { gear_step(&S, S.gamma_cur, t[0]); });
+        if (!ok || S.done) break;
+        // K2, two rows a thread and step
+        const float a = (float)S.alpha, b = (float)S.beta;
+        const bool reset = S.y_reset != 0;
+        v[0] = v[1] = 0.0;
+        auto update = [&](float &r, float dd, float w, float &p, float &s, float &y, float &u) {
+            p = r / dd + b * p;
+            s = w + b * s;
+            y = y + a * p;
+            r = r - a * s;
+            u = r / dd;
+            v[0] += (double)r * (double)u;
+            v[1] += (double)r * (double)r;
+        };
+        for (int c = tid; c < n / 2; c += nthreads) {
+            float2 r = reinterpret_cast<const float2 *>(B.r)[c], p = reinterpret_cast<const float2 *>(B.p)[c];
+            float2 s = reinterpret_cast<const float2 *>(B.s)[c], u;
+            float2 y = reset ? make_float2(0.0f, 0.0f) : reinterpret_cast<const float2 *>(B.y)[c];
+            const float2 w = reinterpret_cast<const float2 *>(B.w)[c], dd = reinterpret_cast<const float2 *>(B.D)[c];
+            update(r.x, dd.x, w.x, p.x, s.x, y.x, u.x);
+            update(r.y, dd.y, w.y, p.y, s.y, y.y, u.y);
+            reinterpret_cast<float2 *>(B.p)[c] = p;
+            reinterpret_cast<float2 *>(B.s)[c] = s;
+            reinterpret_cast<float2 *>(B.y)[c] = y;
+            reinterpret_cast<float2 *>(B.r)[c] = r;
+            reinterpret_cast<float2 *>(B.u)[c] = u;
+        }
+        if ((n & 1) && tid == 0) {
+            const int i = n - 1;
+            float r = B.r[i], p = B.p[i], s = B.s[i], y = reset ? 0.0f : B.y[i], u;
+            update(r, B.D[i], B.w[i], p, s, y, u);
+            B.p[i] = p;
+            B.s[i] = s;
+            B.y[i] = y;
+            B.r[i] = r;
+            B.u[i] = u;
+        }
+        ok = G.sum(v, [&](const double *t) {
+            S.gamma_cur = t[0];
+            S.rr_cur = t[1];
+            S.ru_due = gear_check(&S, t[1]) ? 1 : 0;
+        });
+        if (!ok || S.done || !S.ru_due) continue;
+        // R0, R1
+        for (int i = tid; i < n; i += nthreads) B.x[i] += (double)B.y[i];
+        if (!(ok = G.sync())) break;
+        v3[0] = v3[1] = v3[2] = 0.0;
+        for (int s = warp; s < nsl; s += nwarps) {
+            const int pos = s * 32 + lane;
+            const int32_t row = Q.perm[pos];
+            const double *x = B.x;
+            const double acc = q16_row64_with(Q, s, lane, Q.len[pos], Q.split[pos], Q.base0[pos], Q.base1[pos],
+                                              [x](int32_t c) { return x[c]; });
+            if (row >= 0) {
+                const double rt = B.b[row] - acc;
+                const float rf = (float)rt, uf = rf / B.D[row];
+                B.r[row] = rf;
+                B.u[row] = uf;
+                v3[0] += rt * rt;
+                v3[1] += (double)rf * (double)uf;
+                v3[2] += (double)rf * (double)rf;
+            }
+        }
+        ok = G.sum(v3, [&](const double *t) { gear_updated(&S, t); });
+    }
+    if (threadIdx.x == 0 && (blockIdx.x == 0 || !ok)) {
+        if (!ok) {
+            S.done = 1;
+            S.status = GEAR_PASS_LIMIT;
+        }
+        for (int i = 0; i < (int)(sizeof(GearState) / 4); i++)
+            reinterpret_cast<unsigned *>(B.st)[i] = reinterpret_cast<const volatile unsigned *>(&S)[i];
+    }
+}
+
+cudaError_t launch_gear_coop(const GearBuffers &B, const Q16View &Q, int unroll, double *exchange, cudaStream_t s) {
+    auto kernel = unroll == 2 ? gear_coop_kernel<2> : gear_coop_kernel<1>;
+    int dev = 0, coop = 0, sms = 0, per_sm = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kGearCoopThreads, 0);
+    if (e != cudaSuccess) return e;
+    int grid = sms * per_sm < kCoopMostBlocks ? sms * per_sm : kCoopMostBlocks;
+    if (!coop || grid < 1) return cudaErrorNotSupported;
+    GearBuffers b = B;
+    Q16View q = Q;
+    void *args[] = {(void *)&q, (void *)&b, (void *)&exchange};
+    return cudaLaunchCooperativeKernel((const void *)kernel, dim3(grid), dim3(kGearCoopThreads), args, 0, s);
 }
 
 // One pass of the graph loop is over: stop when done, or when the passes

@@ -69,4 +69,9 @@ cudaError_t launch_gear_fold(const GearBuffers &B, cudaStream_t s);
 cudaError_t build_pcg_loop_graph(cudaStream_t stream, void (*body)(void *ctx, cudaStream_t s), void *ctx,
                                  PcgState *st, bool plain, cudaGraphExec_t *exec);
 
+// The iterations from the state in B.st on the q16 layout as one cooperative
+// kernel (exchange: coop_exchange_doubles(), zero before the launch);
+// cudaErrorNotSupported where the device cannot launch it.
+cudaError_t launch_gear_coop(const GearBuffers &B, const Q16View &Q, int unroll, double *exchange, cudaStream_t s);
+
 }  // namespace phgb

@@ -43,7 +43,7 @@ mixed_coop_kernel(const MixedRun R) {
     __shared__ CoopShared sh;
     __shared__ MixedScalars S;
     __shared__ int next_unit;
-    CoopGrid G(R.exchange, &sh);
+    CoopGrid<> G(R.exchange, &sh);
     const int t = threadIdx.x;
     const unsigned n = (unsigned)R.A.n;
     const int m = coop_places(n);

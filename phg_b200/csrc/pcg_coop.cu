@@ -47,7 +47,7 @@ pcg_coop_kernel(const PcgRun R) {
     __shared__ CoopShared sh;
     __shared__ PcgScalars S;
     __shared__ int next_unit;
-    CoopGrid G(R.exchange, &sh);
+    CoopGrid<> G(R.exchange, &sh);
     const int t = threadIdx.x;
     const unsigned n = (unsigned)R.A.n;
     const int m = coop_places(n);
