@@ -1700,7 +1700,7 @@ int pcg_one_kernel(phgGpuSystem *s, const double *drhs, double rtol, double btol
     if (entries < 0) return 0;
     CHECK_RC(coop_buffers(s, entries));
     const PcgRun run{CsrView{n, s->rp.p, s->ci.p, s->va.p}, s->nnz, s->coop_cols.p, s->coop_vals.p, s->x.p, s->p.p,
-                     drhs, s->diag.p, rtol, btol, atol, maxit, dhist, s->coop_xch.p, s->st.p};
+                     s->Ap.p, s->r.p, drhs, s->diag.p, rtol, btol, atol, maxit, dhist, s->coop_xch.p, s->st.p};
     CK(launch_pcg_coop(run, s->stream));
     s->launches += 1;
     CK(cudaMemcpyAsync(s->h_st, s->st.p, sizeof(PcgState), cudaMemcpyDeviceToHost, s->stream));

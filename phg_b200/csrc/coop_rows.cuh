@@ -35,6 +35,11 @@ __device__ __forceinline__ int coop_places(int64_t n) {
     return 32 * (int)(((n + 31) / 32 - blockIdx.x + gridDim.x - 1) / gridDim.x);
 }
 
+// Entry c of a vector: a pointer (read with plain loads: other blocks write it
+// between barriers) or a function of the column.
+template <class V> __device__ __forceinline__ V entry_of(const V *x, int32_t c) { return x[c]; }
+template <class F> __device__ __forceinline__ auto entry_of(const F &f, int32_t c) -> decltype(f(c)) { return f(c); }
+
 template <int H>
 struct CoopRows {
     int slices;             // of the block; its slice k is slice blockIdx.x + gridDim.x * k
@@ -106,13 +111,13 @@ struct CoopRows {
     }
 
     // y[place] = (A x)_row for the block's places (shared memory, zero in the
-    // padding), values `vals` in step order.  x is read with plain loads: other
-    // blocks write it between barriers.  All threads call it, with y free to
-    // write; y is complete when it returns.  ORDERED: each row's sum takes its
+    // padding), values `vals` in step order, x a vector or a function of the column
+    // (entry_of).  All threads call it, with y free to write; y is complete
+    // when it returns.  ORDERED: each row's sum takes its
     // entries in CSR order, one by one, whatever H (the sums of the launched
     // SELL products); otherwise the lanes' sums are added.
-    template <bool ORDERED, class V>
-    __device__ __forceinline__ void product(const V *vals, const V *x, V *y) const {
+    template <bool ORDERED, class V, class X>
+    __device__ __forceinline__ void product(const V *vals, X x, V *y) const {
         const int lane = threadIdx.x & 31, units = H * slices;
         for (int unit = threadIdx.x >> 5; unit < units;) {
             const int place = place_of(unit, lane);
@@ -131,8 +136,8 @@ struct CoopRows {
     // f(place, (A x)_row) in one lane for each of the block's places: the
     // product (ordered) without a place to keep it, the units dealt to the
     // warps in turn.
-    template <class V, class F>
-    __device__ __forceinline__ void product_each(const V *vals, const V *x, F f) const {
+    template <class V, class X, class F>
+    __device__ __forceinline__ void product_each(const V *vals, X x, F f) const {
         const int lane = threadIdx.x & 31;
         for (int unit = threadIdx.x >> 5; unit < H * slices; unit += kCoopWarps) {
             const int place = place_of(unit, lane);
@@ -145,8 +150,8 @@ private:
     // Sum of the lane's row, of length l, in every lane of the row; the
     // unit's entries start at `at`.  FP32 entries are loaded a batch ahead of
     // the gathers they feed (FP64 ones would not fit the registers).
-    template <bool ORDERED, class V>
-    __device__ __forceinline__ V row_sum(const V *vals, const V *x, int at, int l) const {
+    template <bool ORDERED, class V, class X>
+    __device__ __forceinline__ V row_sum(const V *vals, X x, int at, int l) const {
         constexpr int U = 8;
         constexpr bool ahead = sizeof(V) == 4;
         const int lane = threadIdx.x & 31, mine = own(l, lane);
@@ -183,7 +188,7 @@ private:
             }
             V xv[U];
 #pragma unroll
-            for (int u = 0; u < U; u++) xv[u] = c[u] >= 0 ? x[c[u]] : (V)0;
+            for (int u = 0; u < U; u++) xv[u] = c[u] >= 0 ? entry_of(x, c[u]) : (V)0;
             if constexpr (ORDERED && H > 1) {
 #pragma unroll
                 for (int u = 0; u < U; u++)

@@ -9,11 +9,14 @@
 //   product    w = A p, and p.w                              (sum)
 //   update     r -= alpha w, z = r / diag, ||r||^2 and r.z    (sum; x += alpha p
 //              runs behind the barrier)
+// Where a barrier costs more than gathers (FUSED, small systems), z goes through
+// L2 too and the product gathers z + beta p from z and the last direction, so
+// that the direction needs no barrier of its own; the values are the same.
 // What bounds it: at 1,000 to 40,000 rows the three barriers, about 1.4 us each,
 // and the latency of the phases between them; from 100,000 rows on the product,
 // which reads the matrix from L2 (up to some 10 million entries) at the rate
 // its gathers allow.  Time per iteration against the same recurrence as three
-// launches in a graph loop: P1 1,331 rows 6.7 us (16.3), P1 36k 7.9 (18.9), P1
+// launches in a graph loop: P1 1,331 rows 6.7 us (16.3), P1 36k 6.9 (18.9), P1
 // 133k 10.4 (20.7), P1 389k 18.5 (33.3), P2 69k 11.3 (23.4), P2 250k 22.5
 // (37.4), P2 531k 38.5 (58.5), P3 227k 30.8 (52.2); and a solve needs no tuned
 // layout, no graph and one host wait: 71 us instead of 180 before the first
@@ -40,7 +43,7 @@ struct PcgScalars {
 
 __device__ __forceinline__ bool is_zero(double a) { return fabs(a) < 10.0 * DBL_MIN; }   // utils.h:451
 
-template <int H>
+template <int H, bool FUSED>
 __global__ void __launch_bounds__(kCoopThreads, 1)
 pcg_coop_kernel(const PcgRun R) {
     extern __shared__ double s_vec[];
@@ -101,13 +104,17 @@ pcg_coop_kernel(const PcgRun R) {
     __syncthreads();
     // r = b - A x, or b when x = 0
     if (S.nonzero) {
-        L.template product<false>(R.vals, R.x, sw);
+        L.template product<false>(R.vals, (const double *)R.x, sw);
         for (int i = t; i < m; i += kCoopThreads) sr[i] -= sw[i];
     }
     v[0] = v[1] = 0.0;
     for (int i = t; i < m; i += kCoopThreads) {
         const double ri = sr[i], zi = ri / sD[i];
         sw[i] = zi;
+        if (FUSED && L.row(i) < n) {
+            R.z[L.row(i)] = zi;
+            R.p[L.row(i)] = 0.0;
+        }
         v[0] += ri * ri;
         v[1] += ri * zi;
     }
@@ -124,18 +131,35 @@ pcg_coop_kernel(const PcgRun R) {
         if (!isfinite(s[1])) S.status = kStatusBadStart;
         S.run = S.status == PCG_RUNNING && res > tol && R.maxit > 0;
     });
+    // (`start` with a beta of 0 would do as in FUSED, but the compiler then orders
+    // the product's gathers worse: P2 531k rows 45.9 us instead of 38.4)
     bool start = true;
+    double *from = R.p, *to = R.p2;   // FUSED: the last direction and the next
     while (ok && S.run) {
         const double beta = S.beta;
-        for (int i = t; i < m; i += kCoopThreads) {
-            const double pi = start ? sw[i] : beta * sp[i] + sw[i];
-            sp[i] = pi;
-            if (L.row(i) < n) R.p[L.row(i)] = pi;
+        if constexpr (FUSED) {
+            const double *pold = from, *zold = R.z;
+            for (int i = t; i < m; i += kCoopThreads) {
+                const double pi = beta * sp[i] + sw[i];
+                sp[i] = pi;
+                if (L.row(i) < n) to[L.row(i)] = pi;
+            }
+            __syncthreads();
+            L.template product<false>(R.vals, [=](int32_t c) { return beta * pold[c] + zold[c]; }, sw);
+            double *other = from;
+            from = to;
+            to = other;
+        } else {
+            for (int i = t; i < m; i += kCoopThreads) {
+                const double pi = start ? sw[i] : beta * sp[i] + sw[i];
+                sp[i] = pi;
+                if (L.row(i) < n) R.p[L.row(i)] = pi;
+            }
+            start = false;
+            if (!(ok = G.sync())) break;
+            L.template product<false>(R.vals, (const double *)R.p, sw);
         }
-        start = false;
-        if (!(ok = G.sync())) break;
         d[0] = 0.0;
-        L.template product<false>(R.vals, R.p, sw);
         for (int i = t; i < m; i += kCoopThreads) d[0] += sp[i] * sw[i];
         ok = G.sum(d, [&](const double *s) {
             if (s[0] == 0.0) {
@@ -152,6 +176,7 @@ pcg_coop_kernel(const PcgRun R) {
             const double ri = sr[i] - alpha * sw[i], zi = ri / sD[i];
             sr[i] = ri;
             sw[i] = zi;
+            if (FUSED && L.row(i) < n) R.z[L.row(i)] = zi;
             v[0] += ri * ri;
             v[1] += ri * zi;
         }
@@ -189,6 +214,11 @@ pcg_coop_kernel(const PcgRun R) {
 }
 
 constexpr int64_t kRowBytes = 4 * sizeof(double);   // r, w / z, p, diagonal
+// Entries up to which the product forms the direction from the two vectors it
+// gathers, saving a barrier: us per iteration with / without, P1 9k rows 6.8 /
+// 7.7, P1 36k (430,000 entries) 6.9 / 7.9, P2 9k 8.5 / 9.2, P1 133k (1.7 million)
+// 10.3 / 10.6, P2 69k (1.6 million) 11.4 / 11.3, P3 51k (1.9 million) 16.1 / 15.2.
+constexpr int64_t kFusedEntries = 1500000;
 
 }  // namespace
 
@@ -202,10 +232,17 @@ int64_t pcg_coop_entries(int64_t n, int64_t nnz) {
 cudaError_t launch_pcg_coop(const PcgRun &R, cudaStream_t s) {
     CoopSplit sp;
     if (!coop_split(R.A.n, R.nnz, kRowBytes, 0, 4, &sp)) return cudaErrorCooperativeLaunchTooLarge;
+    if (R.nnz <= kFusedEntries) {
+        switch (sp.lanes) {
+        case 1: return coop_launch(pcg_coop_kernel<1, true>, R, sp, s);
+        case 2: return coop_launch(pcg_coop_kernel<2, true>, R, sp, s);
+        default: return coop_launch(pcg_coop_kernel<4, true>, R, sp, s);
+        }
+    }
     switch (sp.lanes) {
-    case 1: return coop_launch(pcg_coop_kernel<1>, R, sp, s);
-    case 2: return coop_launch(pcg_coop_kernel<2>, R, sp, s);
-    default: return coop_launch(pcg_coop_kernel<4>, R, sp, s);
+    case 1: return coop_launch(pcg_coop_kernel<1, false>, R, sp, s);
+    case 2: return coop_launch(pcg_coop_kernel<2, false>, R, sp, s);
+    default: return coop_launch(pcg_coop_kernel<4, false>, R, sp, s);
     }
 }
 

@@ -4,14 +4,14 @@
 
 namespace phgb {
 
-// One solve of A x = b from the initial guess in x: p (n) is the direction
-// the product gathers, the other vectors stay on chip.
+// One solve of A x = b from the initial guess in x: p (and for small systems p2
+// and z) are what the product gathers, the other vectors stay on chip.
 struct PcgRun {
     CsrView A;
     int64_t nnz;
     int32_t *cols;       // the blocks' copy of the matrix: pcg_coop_entries() each
     double *vals;
-    double *x, *p;
+    double *x, *p, *p2, *z;   // n each
     const double *b, *D;
     double rtol, btol, atol;
     int maxit;
