@@ -272,8 +272,9 @@ int phgGpuSolverPCGMixed(phgGpuSystem *sys, double rtol, double btol,
 			 int *nupdates);
 
 /* The SpMV layout the autotuner chose for the current matrix (no
- * counterpart in the reference): at the first solve or product for a matrix
- * shape it times CSR with 4/8/16/32 lanes per row and SELL-C-sigma (32-row
+ * counterpart in the reference): at the first product or launched solve for a
+ * matrix shape (a solve that runs as one kernel needs no layout; after one, this
+ * call makes the choice) it times CSR with 4/8/16/32 lanes per row and SELL-C-sigma (32-row
  * slices, rows sorted by length in 256-row windows) with 2/4/8-fold
  * unrolling, and keeps the fastest.  kind: 0 = CSR (param = lanes per row),
  * 1 = SELL (param = unroll), 2 = q16 (param = 1; the 16-bit-column layout
