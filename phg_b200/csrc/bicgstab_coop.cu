@@ -54,7 +54,7 @@ bicg_coop_kernel(const BicgRun R) {
         if (in) {
             v3[0] += fabs(R.x[row]);
             v3[1] += bi * bi;
-            if (R.A.rp[row + 1] - R.A.rp[row] > kCoopMaxRowLen) v3[2] = 1.0;
+            if (R.A.rp[row + 1] - R.A.rp[row] > R.max_row) v3[2] = 1.0;
         }
     }
     bool ok = G.sum(v3, [&](const double *s) {
@@ -227,18 +227,19 @@ bicg_coop_kernel(const BicgRun R) {
     }
 }
 
+constexpr int kSpare = 64;   // coop_max_row
 constexpr int64_t kRowBytes = 6 * sizeof(double);   // r / s, rh, p, v, t, diagonal
 
 }  // namespace
 
 int64_t bicg_coop_entries(int64_t n, int64_t nnz) {
     CoopSplit sp;
-    return coop_split(n, nnz, kRowBytes, 0, 4, &sp) ? nnz : -1;
+    return coop_split(n, nnz, kRowBytes, 0, 4, kSpare, &sp) ? nnz : -1;
 }
 
 cudaError_t launch_bicg_coop(const BicgRun &R, cudaStream_t s) {
     CoopSplit sp;
-    if (!coop_split(R.A.n, R.nnz, kRowBytes, 0, 4, &sp)) return cudaErrorCooperativeLaunchTooLarge;
+    if (!coop_split(R.A.n, R.nnz, kRowBytes, 0, 4, kSpare, &sp)) return cudaErrorCooperativeLaunchTooLarge;
     switch (sp.lanes) {
     case 1: return coop_launch(bicg_coop_kernel<1>, R, sp, s);
     case 2: return coop_launch(bicg_coop_kernel<2>, R, sp, s);

@@ -1355,7 +1355,7 @@ static int mixed_one_kernel(phgGpuSystem *s, double rtol, double btol, double at
     CHECK_RC(s->mixed_out.ensure(1));
     if (s->h_mixed == nullptr) CK(cudaMallocHost((void **)&s->h_mixed, sizeof(MixedResult)));
     const MixedRun run{CsrView{n, s->rp.p, s->ci.p, s->va.p}, s->nnz, s->coop_cols.p, s->coop_vals32.p, s->coop_vals.p,
-                       s->x.p, s->u32.p, s->rhs.p, s->diag.p, rtol, btol, atol, 0.1, maxit, s->coop_xch.p,
+                       s->x.p, s->u32.p, s->rhs.p, s->diag.p, rtol, btol, atol, 0.1, maxit, s->coop_xch.p, 0,
                        s->mixed_out.p};
     CK(launch_mixed_coop(run, s->stream));
     s->launches += 1;
@@ -1700,7 +1700,7 @@ int pcg_one_kernel(phgGpuSystem *s, const double *drhs, double rtol, double btol
     if (entries < 0) return 0;
     CHECK_RC(coop_buffers(s, entries));
     const PcgRun run{CsrView{n, s->rp.p, s->ci.p, s->va.p}, s->nnz, s->coop_cols.p, s->coop_vals.p, s->x.p, s->p.p,
-                     s->Ap.p, s->r.p, drhs, s->diag.p, rtol, btol, atol, maxit, dhist, s->coop_xch.p, s->st.p};
+                     s->Ap.p, s->r.p, drhs, s->diag.p, rtol, btol, atol, maxit, dhist, s->coop_xch.p, 0, s->st.p};
     CK(launch_pcg_coop(run, s->stream));
     s->launches += 1;
     CK(cudaMemcpyAsync(s->h_st, s->st.p, sizeof(PcgState), cudaMemcpyDeviceToHost, s->stream));
@@ -1829,7 +1829,8 @@ int bicg_one_kernel(phgGpuSystem *s, double rtol, double btol, double atol, int 
     CHECK_RC(s->bicg_st.ensure(1));
     if (s->h_bst == nullptr) CK(cudaMallocHost((void **)&s->h_bst, sizeof(BicgState)));
     const BicgRun run{CsrView{n, s->rp.p, s->ci.p, s->va.p}, s->nnz, s->coop_cols.p, s->coop_vals.p, s->x.p, s->p.p,
-                      s->Ap.p, s->rhs.p, s->diag.p, rtol, btol, atol, maxit, dhist, s->coop_xch.p, s->bicg_st.p};
+                      s->Ap.p, s->rhs.p, s->diag.p, rtol, btol, atol, maxit, dhist, s->coop_xch.p, 0,
+                      s->bicg_st.p};
     CK(launch_bicg_coop(run, s->stream));
     s->launches += 1;
     CK(cudaMemcpyAsync(s->h_bst, s->bicg_st.p, sizeof(BicgState), cudaMemcpyDeviceToHost, s->stream));
@@ -2011,7 +2012,7 @@ static int gmres_impl(phgGpuSystem *s, int restart, int augk, double rtol, doubl
         double *Z1 = flex ? F1 + (int64_t)(restart + 1) * stride : nullptr;
         if (flex) CK(cudaMemsetAsync(Z1, 0, sizeof(double) * (size_t)stride * augk, s->stream));
         const GmresRun run{CsrView{n, s->rp.p, s->ci.p, s->va.p}, s->nnz, s->coop_cols.p, s->coop_vals.p, s->x.p, s->rhs.p,
-                           s->diag.p, V, F1, Z1, stride, rtol, btol, atol, maxit, mk, flex ? augk : -1, s->coop_xch.p,
+                           s->diag.p, V, F1, Z1, stride, rtol, btol, atol, maxit, mk, flex ? augk : -1, s->coop_xch.p, 0,
                            s->gm_st.p};
         CK(launch_gmres_coop(run, s->stream));
         s->launches += 1;

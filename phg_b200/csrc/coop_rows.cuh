@@ -22,7 +22,7 @@
 
 namespace phgb {
 
-constexpr int kCoopMaxRowLen = 1024;   // longer rows would be a few lanes' serial work
+constexpr int kCoopMaxRowLen = 1024;   // of any of these solvers (coop_max_row)
 
 // Shared memory of the row bookkeeping of a block with that many slices: the
 // rows' lengths and each unit's first entry.
@@ -255,9 +255,36 @@ inline int coop_lanes(int64_t slices, int64_t n, int64_t nnz, int most) {
     return h;
 }
 
-// The launch of a one-kernel solver: blocks, lanes a row and shared memory
-// (`fixed_bytes`, `row_bytes` of vectors a row, and the row bookkeeping); false
-// when it is too large.
+// The longest row an FP64 solver takes.  A row is its lanes' serial work, some
+// 0.14 us an entry and lane while the other blocks wait, where the launched
+// products share it among up to 32 lanes: so it may cost what the launches cost
+// and what the blocks' average product hides.  `spare` is the first in entries
+// a lane, an entry of a block's product counts 1/128 of one.  Measured us per
+// iteration, 7 entries a row and one row of L, one kernel / launched:
+// PCG (spare 72)          L = 7        100         200         500
+//   2.2k rows         6.5 / 15.8  20.6 / 16.0  34.6 / 17.1  80.4 / 19.5
+//   39k               6.6 / 15.1  18.8 / 17.8  32.1 / 19.8  71.7 / 23.3
+//   373k             12.8 / 23.2  19.9 / 28.0  30.0 / 33.3  59.2 / 46.3
+// BiCGstab (64, two products an iteration)
+//   39k              14.1 / 29.8  33.0 / 30.5  53.1 / 34.4   114 / 47.7
+//   373k             24.3 / 48.4  40.6 / 57.7  63.6 / 65.8   131 / 77.2
+// GMRES, restart 10 (176)
+//   2.2k             20.5 / 40.8  31.6 / 42.9  44.0 / 41.6  82.7 / 45.5
+//   39k              20.7 / 43.0  31.1 / 45.5  42.6 / 45.6  77.2 / 53.0
+//   373k             33.2 / 58.2  42.2 / 63.3  54.5 / 68.8  95.0 / 76.2
+// Meshes of random points stay below it: PCG, P3 on 3,000 points (rows of up to 371
+// entries, 47 on average, four lanes) 22.8 / 29.4, on 9,000 (two lanes) 49.3 / 65.9.
+// The mixed solver's launched FP32 products give a row one lane too, and it has
+// no limit but kCoopMaxRowLen: L = 1000, 2.2k rows 72.6 / 93.7, 373k 87.8 / 237.
+inline int coop_max_row(int64_t nnz, int blocks, int lanes, int spare) {
+    const int64_t most = lanes * (spare + nnz / blocks / 128);
+    return most < kCoopMaxRowLen ? (int)most : kCoopMaxRowLen;
+}
+
+// The launch of a one-kernel solver: blocks, lanes a row, longest row and shared
+// memory (`fixed_bytes`, `row_bytes` of vectors a row, and the row bookkeeping);
+// false when it is too large.  `spare`: see coop_max_row, 0 for no limit of the
+// kind.
 //
 // Shared memory a solve takes at most: what it takes the L1 cache loses, and
 // the product's gathers need that.  With 122 KB a block (P2, 531k rows) an
@@ -269,11 +296,11 @@ constexpr int64_t kCoopMaxSmem = 136 * 1024;
 constexpr int64_t kCoopBlockWork = 4096;
 
 struct CoopSplit {
-    int blocks = 0, lanes = 1;
+    int blocks = 0, lanes = 1, max_row = 0;
     int64_t smem = 0;
 };
 
-inline bool coop_split(int64_t n, int64_t nnz, int64_t row_bytes, int64_t fixed_bytes, int most_lanes,
+inline bool coop_split(int64_t n, int64_t nnz, int64_t row_bytes, int64_t fixed_bytes, int most_lanes, int spare,
                        CoopSplit *out) {
     int dev = 0, coop = 0, sms = 0, most = 0;
     if (cudaGetDevice(&dev) != cudaSuccess ||
@@ -292,16 +319,19 @@ inline bool coop_split(int64_t n, int64_t nnz, int64_t row_bytes, int64_t fixed_
     const int64_t per = ceil_div(slices, G);
     out->blocks = (int)G;
     out->lanes = coop_lanes(per, n, nnz, most_lanes);
+    out->max_row = spare > 0 ? coop_max_row(nnz, out->blocks, out->lanes, spare) : kCoopMaxRowLen;
     out->smem = fixed_bytes + 32 * per * row_bytes + coop_rows_bytes(per, out->lanes);
     return out->smem <= kCoopMaxSmem && out->smem <= most - 4096;   // 4 KB of static shared memory at most
 }
 
-// Cooperative launch of kernel(run) with that split.
+// Cooperative launch of kernel(run) with that split, whose longest row goes to
+// run.max_row.
 template <class Run>
 inline cudaError_t coop_launch(void (*kernel)(Run), const Run &run, const CoopSplit &sp, cudaStream_t s) {
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCoopMaxSmem);
     if (e != cudaSuccess) return e;
     Run r = run;
+    r.max_row = sp.max_row;
     void *args[] = {(void *)&r};
     return cudaLaunchCooperativeKernel((const void *)kernel, dim3(sp.blocks), dim3(kCoopThreads), args, (size_t)sp.smem, s);
 }

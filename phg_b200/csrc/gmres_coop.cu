@@ -113,7 +113,7 @@ gmres_coop_kernel(const GmresRun R) {
         sD[i] = row < n ? R.D[row] : 1.0;
         if (row < n) {
             v2[0] += R.b[row] * R.b[row];
-            if (R.A.rp[row + 1] - R.A.rp[row] > kCoopMaxRowLen) v2[1] = 1.0;
+            if (R.A.rp[row + 1] - R.A.rp[row] > R.max_row) v2[1] = 1.0;
         }
     }
     for (int i = t; i < R2 * R2 + 4 * R2; i += kCoopThreads) sH[i] = 0.0;
@@ -259,18 +259,19 @@ gmres_coop_kernel(const GmresRun R) {
     }
 }
 
+constexpr int kSpare = 176;   // coop_max_row
 constexpr int64_t kRowBytes = 3 * sizeof(double);   // w, z, diagonal
 
 }  // namespace
 
 int64_t gmres_coop_entries(int64_t n, int64_t nnz, int restart) {
     CoopSplit sp;
-    return coop_split(n, nnz, kRowBytes, 8 * dense_doubles(restart), 4, &sp) ? nnz : -1;
+    return coop_split(n, nnz, kRowBytes, 8 * dense_doubles(restart), 4, kSpare, &sp) ? nnz : -1;
 }
 
 cudaError_t launch_gmres_coop(const GmresRun &R, cudaStream_t s) {
     CoopSplit sp;
-    if (!coop_split(R.A.n, R.nnz, kRowBytes, 8 * dense_doubles(R.mk + (R.augk >= 0 ? R.augk : 0)), 4, &sp))
+    if (!coop_split(R.A.n, R.nnz, kRowBytes, 8 * dense_doubles(R.mk + (R.augk >= 0 ? R.augk : 0)), 4, kSpare, &sp))
         return cudaErrorCooperativeLaunchTooLarge;
     switch (sp.lanes) {
     case 1: return coop_launch(gmres_coop_kernel<1>, R, sp, s);

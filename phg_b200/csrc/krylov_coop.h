@@ -19,6 +19,7 @@ struct BicgRun {
     int maxit;
     double *hist;        // optional: ||r|| after each iteration
     double *exchange;    // coop_exchange_doubles(), zero before the launch
+    int max_row;         // a longer row declines the solve; set by the launch
     BicgState *st;       // out: nits, residual, status (BICG_*)
 };
 
@@ -36,6 +37,7 @@ struct GmresRun {
     double rtol, btol, atol;
     int maxit, mk, augk; // steps of the first cycle, augmenting corrections
     double *exchange;
+    int max_row;         // a longer row declines the solve; set by the launch
     GmresState *st;      // out: nits, residual, status (GMRES_*, kStatus*)
 };
 

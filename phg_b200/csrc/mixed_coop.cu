@@ -60,7 +60,7 @@ mixed_coop_kernel(const MixedRun R) {
             const double bi = R.b[row];
             v3[0] += fabs(R.x[row]);
             v3[1] += bi * bi;
-            if (R.A.rp[row + 1] - R.A.rp[row] > kCoopMaxRowLen) v3[2] = 1.0;
+            if (R.A.rp[row + 1] - R.A.rp[row] > R.max_row) v3[2] = 1.0;
         }
     }
     bool ok = G.sum(v3, [&](const double *s) {
@@ -237,12 +237,12 @@ constexpr int64_t kMaxEntries = 10000000;
 
 int64_t mixed_coop_entries(int64_t n, int64_t nnz) {
     CoopSplit sp;
-    return nnz <= kMaxEntries && coop_split(n, nnz, kRowBytes, 0, 2, &sp) ? nnz : -1;
+    return nnz <= kMaxEntries && coop_split(n, nnz, kRowBytes, 0, 2, 0, &sp) ? nnz : -1;
 }
 
 cudaError_t launch_mixed_coop(const MixedRun &R, cudaStream_t s) {
     CoopSplit sp;
-    if (!coop_split(R.A.n, R.nnz, kRowBytes, 0, 2, &sp)) return cudaErrorCooperativeLaunchTooLarge;
+    if (!coop_split(R.A.n, R.nnz, kRowBytes, 0, 2, 0, &sp)) return cudaErrorCooperativeLaunchTooLarge;
     return sp.lanes == 1 ? coop_launch(mixed_coop_kernel<1>, R, sp, s) : coop_launch(mixed_coop_kernel<2>, R, sp, s);
 }
 

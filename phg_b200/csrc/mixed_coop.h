@@ -23,6 +23,7 @@ struct MixedRun {
     double rtol, btol, atol, delta;
     int maxit;
     double *exchange;    // coop_exchange_doubles(), zero before the launch
+    int max_row;         // a longer row declines the solve; set by the launch
     MixedResult *out;
 };
 

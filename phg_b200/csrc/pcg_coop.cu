@@ -71,7 +71,7 @@ pcg_coop_kernel(const PcgRun R) {
         if (in) {
             v3[0] += fabs(R.x[row]);
             v3[1] += bi * bi;
-            if (R.A.rp[row + 1] - R.A.rp[row] > kCoopMaxRowLen) v3[2] = 1.0;
+            if (R.A.rp[row + 1] - R.A.rp[row] > R.max_row) v3[2] = 1.0;
         }
     }
     if (!G.sum(v3, [&](const double *s) {
@@ -213,6 +213,7 @@ pcg_coop_kernel(const PcgRun R) {
     }
 }
 
+constexpr int kSpare = 72;   // coop_max_row
 constexpr int64_t kRowBytes = 4 * sizeof(double);   // r, w / z, p, diagonal
 // Entries up to which the product forms the direction from the two vectors it
 // gathers, saving a barrier: us per iteration with / without, P1 9k rows 6.8 /
@@ -226,12 +227,12 @@ int coop_exchange_doubles() { return kCoopDoubles; }
 
 int64_t pcg_coop_entries(int64_t n, int64_t nnz) {
     CoopSplit sp;
-    return coop_split(n, nnz, kRowBytes, 0, 4, &sp) ? nnz : -1;
+    return coop_split(n, nnz, kRowBytes, 0, 4, kSpare, &sp) ? nnz : -1;
 }
 
 cudaError_t launch_pcg_coop(const PcgRun &R, cudaStream_t s) {
     CoopSplit sp;
-    if (!coop_split(R.A.n, R.nnz, kRowBytes, 0, 4, &sp)) return cudaErrorCooperativeLaunchTooLarge;
+    if (!coop_split(R.A.n, R.nnz, kRowBytes, 0, 4, kSpare, &sp)) return cudaErrorCooperativeLaunchTooLarge;
     if (R.nnz <= kFusedEntries) {
         switch (sp.lanes) {
         case 1: return coop_launch(pcg_coop_kernel<1, true>, R, sp, s);

@@ -17,6 +17,7 @@ struct PcgRun {
     int maxit;
     double *hist;        // optional: ||r|| after each iteration, [0] = ||r0||
     double *exchange;    // coop_exchange_doubles(), zero before the launch
+    int max_row;         // a longer row declines the solve; set by the launch
     PcgState *st;        // out: nits, residual, status
 };
 

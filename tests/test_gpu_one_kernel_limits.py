@@ -1,0 +1,80 @@
+"""Which solves run as one cooperative kernel, and that those it leaves go to
+the launched iteration and reach the same solution.  The path is seen in the
+number of kernels the system has launched: one for a solve in one kernel."""
+import numpy as np
+import pytest
+
+from test_gpu_one_kernel import banded_spd, diagonal
+
+pytestmark = pytest.mark.gpu
+
+SOLVERS = ("pcg", "mixed", "bicgstab", "gmres", "flgmres")
+
+
+def solve(s, solver, rtol=1e-9, **kw):
+    """(x, iterations) of one solve by that solver."""
+    if solver == "mixed":
+        return s.solve_pcg_mixed(rtol=rtol, **kw)[:2]
+    kw = dict(rtol=rtol, btol=0.0, atol=0.0, **kw)
+    if solver == "pcg":
+        return s.solve_pcg(**kw)[:2]
+    if solver == "bicgstab":
+        return s.solve_bicgstab(**kw)[:2]
+    if solver == "gmres":
+        return s.solve_gmres(restart=6, **kw)[:2]
+    return s.solve_flgmres(restart=4, augk=2, **kw)[:2]
+
+
+def launches(s, f):
+    """(f(), kernels launched by it)."""
+    before = s.launch_count()
+    out = f()
+    return out, s.launch_count() - before
+
+
+def check(oracle, A, solver, x, rtol=1e-9):
+    """The solution of the oracle's solver (PCG for the SPD solvers), by
+    relative L2 distance 1e3 * rtol as everywhere for these solvers."""
+    ptr, cols, vals, b = A
+    kw = dict(rtol=rtol, btol=0.0, atol=0.0)
+    d = diagonal(ptr, cols, vals)
+    if solver in ("pcg", "mixed"):
+        xo = oracle.pcg(ptr, cols, vals, d, b, **kw)[0]
+    elif solver == "bicgstab":
+        xo = oracle.bicgstab(ptr, cols, vals, d, b, **kw)[0]
+    else:
+        xo = oracle.gmres(ptr, cols, vals, d, b, restart=6, **kw)[0]
+    assert np.linalg.norm(x - xo) <= 1e3 * rtol * np.linalg.norm(xo)
+
+
+def one_long_row(n, length, seed):
+    """banded_spd rows of some seven entries, and row n / 2 with about `length`."""
+    import scipy.sparse as sp
+    ptr, cols, vals, b = banded_spd(n, 3, seed)
+    A = sp.csr_matrix((vals, cols, ptr), shape=(n, n))
+    rng = np.random.default_rng(seed + 1)
+    r = n // 2
+    c = rng.choice(np.setdiff1d(np.arange(n), [r]), length - 7, replace=False)
+    v = np.full(len(c), -1e-3)
+    B = sp.csr_matrix((np.r_[v, v], (np.r_[np.full(len(c), r), c], np.r_[c, np.full(len(c), r)])), shape=(n, n))
+    B = B + sp.diags(np.asarray(abs(B).sum(1)).ravel())
+    A = sp.csr_matrix(A + B)
+    A.sum_duplicates()
+    return A.indptr.astype(np.int64), A.indices.astype(np.int32), A.data.copy(), b
+
+
+@pytest.mark.parametrize("solver", SOLVERS)
+@pytest.mark.parametrize("length", [20, 60, 300, 900, 1100])
+def test_long_row(gpu, oracle, solver, length):
+    """A row far longer than the others is one warp's serial work: the FP64
+    solvers leave such a matrix to the launched products (300 entries and more
+    here), the mixed one, whose launched products are no better at it, from
+    1025 entries on."""
+    A = one_long_row(2500, length, seed=length)
+    longest = int(np.diff(A[0]).max())
+    one = longest <= 1024 if solver == "mixed" else longest < 80
+    with gpu.Solver(0) as s:
+        s.set_matrix(*A)
+        (x, _), k = launches(s, lambda: solve(s, solver))
+        assert (k == 1) == one, (longest, k)
+        check(oracle, A, solver, x)
