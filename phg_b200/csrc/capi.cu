@@ -216,6 +216,7 @@ struct phgGpuSystem_ {
     DevBuf<MixedResult> mixed_out;
     MixedResult *h_mixed = nullptr;
     DevBuf<double> coop_xch;               // exchange memory of the one-kernel solvers
+    unsigned coop_declined = 0;            // those that declined the current matrix (a row too long for them)
     DevBuf<PcgState> st;
     DevBuf<unsigned> ticket;
     DevBuf<int64_t> tmp64;
@@ -446,6 +447,7 @@ void invalidate_layouts(phgGpuSystem *s) {
     s->sell2_valid = false;
     s->q16_valid = false;
     s->q16_fits = false;
+    s->coop_declined = 0;
 }
 
 // Rows sorted by length in 256-row windows (the slices of every SELL layout).
@@ -718,6 +720,19 @@ int coop_buffers(phgGpuSystem *s, int64_t entries) {
     CHECK_RC(s->coop_xch.ensure((size_t)coop_exchange_doubles()));
     CK(cudaMemsetAsync(s->coop_xch.p, 0, sizeof(double) * coop_exchange_doubles(), s->stream));
     return PHG_GPU_OK;
+}
+
+// One-kernel solvers, as bits of coop_declined.
+enum { COOP_PCG = 1, COOP_MIXED = 2, COOP_BICG = 4, COOP_GMRES = 8 };
+
+// The kernel has declined the matrix: later solves of it go to the launched
+// iteration at once, and the copy's memory is given back.
+int coop_decline(phgGpuSystem *s, unsigned solver) {
+    s->coop_declined |= solver;
+    s->coop_cols.release();
+    s->coop_vals.release();
+    s->coop_vals32.release();
+    return 0;
 }
 
 // Whether the caller chose the product layout for the current matrix shape.
@@ -1347,7 +1362,7 @@ int phgGpuMatVec(phgGpuSystem *s, const double *x, double *y) {
 static int mixed_one_kernel(phgGpuSystem *s, double rtol, double btol, double atol, int maxit) {
     const int64_t n = s->n;
     if (s->plan32_set && s->unroll32 != 0 && s->tuned32_n == n && s->tuned32_nnz == s->nnz) return 0;
-    const int64_t entries = mixed_coop_entries(n, s->nnz);
+    const int64_t entries = s->coop_declined & COOP_MIXED ? -1 : mixed_coop_entries(n, s->nnz);
     if (entries < 0) return 0;
     CHECK_RC(coop_buffers(s, entries));
     CHECK_RC(s->coop_vals32.ensure((size_t)entries));
@@ -1361,7 +1376,7 @@ static int mixed_one_kernel(phgGpuSystem *s, double rtol, double btol, double at
     s->launches += 1;
     CK(cudaMemcpyAsync(s->h_mixed, s->mixed_out.p, sizeof(MixedResult), cudaMemcpyDeviceToHost, s->stream));
     CK(cudaStreamSynchronize(s->stream));
-    if (s->h_mixed->status == kStatusDeclined) return 0;
+    if (s->h_mixed->status == kStatusDeclined) return coop_decline(s, COOP_MIXED);
     s->plan_due = s->plan32_due = true;
     return 1;
 }
@@ -1695,8 +1710,7 @@ namespace {
 int pcg_one_kernel(phgGpuSystem *s, const double *drhs, double rtol, double btol, double atol, int maxit,
                    double *dhist) {
     const int64_t n = s->n;
-    if (plan_forced(s)) return 0;
-    const int64_t entries = pcg_coop_entries(n, s->nnz);
+    const int64_t entries = plan_forced(s) || s->coop_declined & COOP_PCG ? -1 : pcg_coop_entries(n, s->nnz);
     if (entries < 0) return 0;
     CHECK_RC(coop_buffers(s, entries));
     const PcgRun run{CsrView{n, s->rp.p, s->ci.p, s->va.p}, s->nnz, s->coop_cols.p, s->coop_vals.p, s->x.p, s->p.p,
@@ -1705,7 +1719,7 @@ int pcg_one_kernel(phgGpuSystem *s, const double *drhs, double rtol, double btol
     s->launches += 1;
     CK(cudaMemcpyAsync(s->h_st, s->st.p, sizeof(PcgState), cudaMemcpyDeviceToHost, s->stream));
     CK(cudaStreamSynchronize(s->stream));
-    if (s->h_st->status == kStatusDeclined) return 0;
+    if (s->h_st->status == kStatusDeclined) return coop_decline(s, COOP_PCG);
     s->plan_due = true;
     return 1;
 }
@@ -1823,7 +1837,7 @@ int pcg_core(phgGpuSystem *s, const double *drhs, double rtol, double btol, doub
 // or 0 when the kernel does not take it (as pcg_one_kernel).
 int bicg_one_kernel(phgGpuSystem *s, double rtol, double btol, double atol, int maxit, double *dhist) {
     const int64_t n = s->n;
-    const int64_t entries = plan_forced(s) ? -1 : bicg_coop_entries(n, s->nnz);
+    const int64_t entries = plan_forced(s) || s->coop_declined & COOP_BICG ? -1 : bicg_coop_entries(n, s->nnz);
     if (entries < 0) return 0;
     CHECK_RC(coop_buffers(s, entries));
     CHECK_RC(s->bicg_st.ensure(1));
@@ -1835,7 +1849,7 @@ int bicg_one_kernel(phgGpuSystem *s, double rtol, double btol, double atol, int 
     s->launches += 1;
     CK(cudaMemcpyAsync(s->h_bst, s->bicg_st.p, sizeof(BicgState), cudaMemcpyDeviceToHost, s->stream));
     CK(cudaStreamSynchronize(s->stream));
-    if (s->h_bst->status == BICG_DECLINED) return 0;
+    if (s->h_bst->status == BICG_DECLINED) return coop_decline(s, COOP_BICG);
     s->plan_due = true;
     return 1;
 }
@@ -2004,7 +2018,8 @@ static int gmres_impl(phgGpuSystem *s, int restart, int augk, double rtol, doubl
     CHECK_RC(s->gm_st.ensure(1));
     if (s->h_gst == nullptr) CK(cudaMallocHost((void **)&s->h_gst, sizeof(GmresState)));
     // as one cooperative kernel, unless it does not take the matrix (as pcg_one_kernel)
-    const int64_t entries = plan_forced(s) ? -1 : gmres_coop_entries(n, s->nnz, restart);
+    const int64_t entries =
+        plan_forced(s) || s->coop_declined & COOP_GMRES ? -1 : gmres_coop_entries(n, s->nnz, restart);
     if (entries >= 0) {
         CHECK_RC(coop_buffers(s, entries));
         CHECK_RC(s->gm_vecs.ensure((size_t)stride * nvec));
@@ -2031,6 +2046,7 @@ static int gmres_impl(phgGpuSystem *s, int restart, int augk, double rtol, doubl
             CK(cudaStreamSynchronize(s->stream));
             return nits;
         }
+        coop_decline(s, COOP_GMRES);
     }
     // ||b|| (solver-phg.c:1071-1075)
     CK(cudaMemsetAsync(s->ticket.p, 0, sizeof(unsigned) * kRedTickets, s->stream));

@@ -78,3 +78,25 @@ def test_long_row(gpu, oracle, solver, length):
         (x, _), k = launches(s, lambda: solve(s, solver))
         assert (k == 1) == one, (longest, k)
         check(oracle, A, solver, x)
+
+
+@pytest.mark.parametrize("solver", SOLVERS)
+def test_declined_matrix_is_remembered(gpu, solver):
+    """The second solve of a matrix the kernel declined launches what a solve
+    on a layout set by the caller does, no attempt before it; a new matrix is
+    looked at again."""
+    A = one_long_row(2500, 1100, seed=3)
+    with gpu.Solver(0) as s:
+        s.set_matrix(*A)
+        solve(s, solver)
+        layout, param, info = s.spmv_plan()
+        _, second = launches(s, lambda: solve(s, solver))
+        if solver == "mixed":
+            s.set_spmv_plan32(info["fp32_layout"], info["fp32_unroll"])
+        else:
+            s.set_spmv_plan(layout, param)
+        solve(s, solver)   # makes the layout's arrays and graph
+        _, forced = launches(s, lambda: solve(s, solver))
+        assert second == forced > 1
+        s.set_matrix(*banded_spd(2000, 3, seed=4))
+        assert launches(s, lambda: solve(s, solver))[1] == 1
