@@ -713,25 +713,44 @@ SpmvPlan make_plan(phgGpuSystem *s, int kind, int param) {
     return P;
 }
 
-// Memory of a one-kernel solve's matrix copy and exchange.
-int coop_buffers(phgGpuSystem *s, int64_t entries) {
-    CHECK_RC(s->coop_cols.ensure((size_t)entries));
-    CHECK_RC(s->coop_vals.ensure((size_t)entries));
-    CHECK_RC(s->coop_xch.ensure((size_t)coop_exchange_doubles()));
-    CK(cudaMemsetAsync(s->coop_xch.p, 0, sizeof(double) * coop_exchange_doubles(), s->stream));
-    return PHG_GPU_OK;
-}
-
 // One-kernel solvers, as bits of coop_declined.
 enum { COOP_PCG = 1, COOP_MIXED = 2, COOP_BICG = 4, COOP_GMRES = 8 };
+
+// Gives a one-kernel solve's matrix copy back.
+void coop_release(phgGpuSystem *s) {
+    s->coop_cols.release();
+    s->coop_vals.release();
+    s->coop_vals32.release();
+}
+
+// Memory of a one-kernel solve's matrix copy (with FP32 values for the mixed
+// one) and exchange.  Returns 1, or 0 when the device has not enough: the
+// launched iteration may have its layout already.
+int coop_buffers(phgGpuSystem *s, int64_t entries, bool mixed) {
+    if (s->coop_cols.ensure((size_t)entries) != PHG_GPU_OK || s->coop_vals.ensure((size_t)entries) != PHG_GPU_OK ||
+        (mixed && s->coop_vals32.ensure((size_t)entries) != PHG_GPU_OK) ||
+        s->coop_xch.ensure((size_t)coop_exchange_doubles()) != PHG_GPU_OK) {
+        coop_release(s);
+        return 0;
+    }
+    CK(cudaMemsetAsync(s->coop_xch.p, 0, sizeof(double) * coop_exchange_doubles(), s->stream));
+    return 1;
+}
+
+// Whether a cooperative launch was refused because its blocks cannot all be
+// resident here: nothing has run, and the launched iteration can solve it.
+bool coop_refused(cudaError_t e) {
+    if (e != cudaErrorCooperativeLaunchTooLarge && e != cudaErrorLaunchOutOfResources && e != cudaErrorNotSupported)
+        return false;
+    cudaGetLastError();
+    return true;
+}
 
 // The kernel has declined the matrix: later solves of it go to the launched
 // iteration at once, and the copy's memory is given back.
 int coop_decline(phgGpuSystem *s, unsigned solver) {
     s->coop_declined |= solver;
-    s->coop_cols.release();
-    s->coop_vals.release();
-    s->coop_vals32.release();
+    coop_release(s);
     return 0;
 }
 
@@ -1356,23 +1375,25 @@ int phgGpuMatVec(phgGpuSystem *s, const double *x, double *y) {
 }
 
 // The mixed solve as one cooperative kernel (mixed_coop.cu) on s->x, its result
-// in s->h_mixed.  Returns 1, or 0 when the kernel does not take it: a matrix
-// whose vectors exceed the SMs' shared memory, a very long row, or an FP32
-// layout the caller asked for (phgGpuSetSpMVPlan32).
+// in s->h_mixed.  Returns 1, or 0 when the kernel does not take it (as
+// pcg_one_kernel), or the caller asked for an FP32 layout
+// (phgGpuSetSpMVPlan32).
 static int mixed_one_kernel(phgGpuSystem *s, double rtol, double btol, double atol, int maxit) {
     const int64_t n = s->n;
     if (s->plan32_set && s->unroll32 != 0 && s->tuned32_n == n && s->tuned32_nnz == s->nnz) return 0;
     const int64_t entries = s->coop_declined & COOP_MIXED ? -1 : mixed_coop_entries(n, s->nnz);
     if (entries < 0) return 0;
-    CHECK_RC(coop_buffers(s, entries));
-    CHECK_RC(s->coop_vals32.ensure((size_t)entries));
+    const int ready = coop_buffers(s, entries, true);
+    if (ready <= 0) return ready;
     CHECK_RC(s->u32.ensure((size_t)n));
     CHECK_RC(s->mixed_out.ensure(1));
     if (s->h_mixed == nullptr) CK(cudaMallocHost((void **)&s->h_mixed, sizeof(MixedResult)));
     const MixedRun run{CsrView{n, s->rp.p, s->ci.p, s->va.p}, s->nnz, s->coop_cols.p, s->coop_vals32.p, s->coop_vals.p,
                        s->x.p, s->u32.p, s->rhs.p, s->diag.p, rtol, btol, atol, 0.1, maxit, s->coop_xch.p, 0,
                        s->mixed_out.p};
-    CK(launch_mixed_coop(run, s->stream));
+    const cudaError_t e = launch_mixed_coop(run, s->stream);
+    if (coop_refused(e)) return 0;
+    CK(e);
     s->launches += 1;
     CK(cudaMemcpyAsync(s->h_mixed, s->mixed_out.p, sizeof(MixedResult), cudaMemcpyDeviceToHost, s->stream));
     CK(cudaStreamSynchronize(s->stream));
@@ -1474,7 +1495,7 @@ int phgGpuSolverPCGMixed(phgGpuSystem *s, double rtol, double btol, double atol,
     // the q16 layout's iterations run as one cooperative kernel, the other
     // layouts' as a graph
     bool one_kernel = q16 && !s->plain_graphs;
-    if (one_kernel) CHECK_RC(s->coop_xch.ensure((size_t)coop_exchange_doubles()));
+    if (one_kernel) one_kernel = s->coop_xch.ensure((size_t)coop_exchange_doubles()) == PHG_GPU_OK;
     auto mixed_graph = [&]() -> int {
         if (s->graph_mixed != nullptr && s->gkey_mixed == key) return PHG_GPU_OK;
         if (s->graph_mixed != nullptr) { cudaGraphExecDestroy(s->graph_mixed); s->graph_mixed = nullptr; }
@@ -1522,7 +1543,7 @@ int phgGpuSolverPCGMixed(phgGpuSystem *s, double rtol, double btol, double atol,
         if (!g.done && one_kernel) {
             CK(cudaMemsetAsync(s->coop_xch.p, 0, sizeof(double) * coop_exchange_doubles(), s->stream));
             const cudaError_t e = launch_gear_coop(B, Q, s->unroll32, s->coop_xch.p, s->stream);
-            if (e == cudaErrorNotSupported) one_kernel = false;
+            if (coop_refused(e)) one_kernel = false;
             else CK(e);
         }
         if (!g.done && !one_kernel) CHECK_RC(mixed_graph());
@@ -1705,17 +1726,21 @@ namespace {
 
 // The solve as one cooperative kernel (pcg_coop.cu), state left in s->h_st.
 // Returns 1, or 0 when the kernel does not take it: a matrix whose vectors
-// exceed the SMs' shared memory, a very long row, or a product layout the
-// caller asked for (phgGpuSetSpMVPlan).
+// exceed the SMs' shared memory, a very long row, a device that cannot hold
+// its copy or its blocks, or a product layout the caller asked for
+// (phgGpuSetSpMVPlan).
 int pcg_one_kernel(phgGpuSystem *s, const double *drhs, double rtol, double btol, double atol, int maxit,
                    double *dhist) {
     const int64_t n = s->n;
     const int64_t entries = plan_forced(s) || s->coop_declined & COOP_PCG ? -1 : pcg_coop_entries(n, s->nnz);
     if (entries < 0) return 0;
-    CHECK_RC(coop_buffers(s, entries));
+    const int ready = coop_buffers(s, entries, false);
+    if (ready <= 0) return ready;
     const PcgRun run{CsrView{n, s->rp.p, s->ci.p, s->va.p}, s->nnz, s->coop_cols.p, s->coop_vals.p, s->x.p, s->p.p,
                      s->Ap.p, s->r.p, drhs, s->diag.p, rtol, btol, atol, maxit, dhist, s->coop_xch.p, 0, s->st.p};
-    CK(launch_pcg_coop(run, s->stream));
+    const cudaError_t e = launch_pcg_coop(run, s->stream);
+    if (coop_refused(e)) return 0;
+    CK(e);
     s->launches += 1;
     CK(cudaMemcpyAsync(s->h_st, s->st.p, sizeof(PcgState), cudaMemcpyDeviceToHost, s->stream));
     CK(cudaStreamSynchronize(s->stream));
@@ -1839,13 +1864,16 @@ int bicg_one_kernel(phgGpuSystem *s, double rtol, double btol, double atol, int 
     const int64_t n = s->n;
     const int64_t entries = plan_forced(s) || s->coop_declined & COOP_BICG ? -1 : bicg_coop_entries(n, s->nnz);
     if (entries < 0) return 0;
-    CHECK_RC(coop_buffers(s, entries));
+    const int ready = coop_buffers(s, entries, false);
+    if (ready <= 0) return ready;
     CHECK_RC(s->bicg_st.ensure(1));
     if (s->h_bst == nullptr) CK(cudaMallocHost((void **)&s->h_bst, sizeof(BicgState)));
     const BicgRun run{CsrView{n, s->rp.p, s->ci.p, s->va.p}, s->nnz, s->coop_cols.p, s->coop_vals.p, s->x.p, s->p.p,
                       s->Ap.p, s->rhs.p, s->diag.p, rtol, btol, atol, maxit, dhist, s->coop_xch.p, 0,
                       s->bicg_st.p};
-    CK(launch_bicg_coop(run, s->stream));
+    const cudaError_t e = launch_bicg_coop(run, s->stream);
+    if (coop_refused(e)) return 0;
+    CK(e);
     s->launches += 1;
     CK(cudaMemcpyAsync(s->h_bst, s->bicg_st.p, sizeof(BicgState), cudaMemcpyDeviceToHost, s->stream));
     CK(cudaStreamSynchronize(s->stream));
@@ -1996,6 +2024,35 @@ int phgGpuSolverPCG(phgGpuSystem *s, double rtol, double btol, double atol, int 
     return nits;
 }
 
+// GMRES_r or FLGMRES_r (as gmres_impl) as one cooperative kernel on s->x, its
+// state in s->h_gst.  Returns 1, or 0 when the kernel does not take it (as
+// pcg_one_kernel).
+static int gmres_one_kernel(phgGpuSystem *s, int mk, int augk, int64_t stride, double rtol, double btol, double atol,
+                            int maxit) {
+    const int64_t n = s->n;
+    const bool flex = augk >= 0;
+    const int restart = flex ? mk + augk : mk;
+    const int64_t entries =
+        plan_forced(s) || s->coop_declined & COOP_GMRES ? -1 : gmres_coop_entries(n, s->nnz, restart);
+    if (entries < 0) return 0;
+    const int ready = coop_buffers(s, entries, false);
+    if (ready <= 0) return ready;
+    double *V = s->gm_vecs.p + stride, *F1 = flex ? s->gm_vecs.p + (int64_t)(restart + 3) * stride : nullptr;
+    double *Z1 = flex ? F1 + (int64_t)(restart + 1) * stride : nullptr;
+    if (flex) CK(cudaMemsetAsync(Z1, 0, sizeof(double) * (size_t)stride * augk, s->stream));
+    const GmresRun run{CsrView{n, s->rp.p, s->ci.p, s->va.p}, s->nnz, s->coop_cols.p, s->coop_vals.p, s->x.p, s->rhs.p,
+                       s->diag.p, V, F1, Z1, stride, rtol, btol, atol, maxit, mk, augk, s->coop_xch.p, 0, s->gm_st.p};
+    const cudaError_t e = launch_gmres_coop(run, s->stream);
+    if (coop_refused(e)) return 0;
+    CK(e);
+    s->launches += 1;
+    CK(cudaMemcpyAsync(s->h_gst, s->gm_st.p, sizeof(GmresState), cudaMemcpyDeviceToHost, s->stream));
+    CK(cudaStreamSynchronize(s->stream));
+    if (s->h_gst->status == kStatusDeclined) return coop_decline(s, COOP_GMRES);
+    s->plan_due = true;
+    return 1;
+}
+
 // GMRES_r (augk < 0) or FLGMRES_r (augk >= 1 augmenting corrections).
 static int gmres_impl(phgGpuSystem *s, int restart, int augk, double rtol, double btol, double atol, int maxit,
                       double *x, double *residual) {
@@ -2017,36 +2074,20 @@ static int gmres_impl(phgGpuSystem *s, int restart, int augk, double rtol, doubl
     const int nvec = (restart + 3) + (flex ? (restart + 1) + augk : 0);
     CHECK_RC(s->gm_st.ensure(1));
     if (s->h_gst == nullptr) CK(cudaMallocHost((void **)&s->h_gst, sizeof(GmresState)));
-    // as one cooperative kernel, unless it does not take the matrix (as pcg_one_kernel)
-    const int64_t entries =
-        plan_forced(s) || s->coop_declined & COOP_GMRES ? -1 : gmres_coop_entries(n, s->nnz, restart);
-    if (entries >= 0) {
-        CHECK_RC(coop_buffers(s, entries));
-        CHECK_RC(s->gm_vecs.ensure((size_t)stride * nvec));
-        double *V = s->gm_vecs.p + stride, *F1 = flex ? s->gm_vecs.p + (int64_t)(restart + 3) * stride : nullptr;
-        double *Z1 = flex ? F1 + (int64_t)(restart + 1) * stride : nullptr;
-        if (flex) CK(cudaMemsetAsync(Z1, 0, sizeof(double) * (size_t)stride * augk, s->stream));
-        const GmresRun run{CsrView{n, s->rp.p, s->ci.p, s->va.p}, s->nnz, s->coop_cols.p, s->coop_vals.p, s->x.p, s->rhs.p,
-                           s->diag.p, V, F1, Z1, stride, rtol, btol, atol, maxit, mk, flex ? augk : -1, s->coop_xch.p, 0,
-                           s->gm_st.p};
-        CK(launch_gmres_coop(run, s->stream));
-        s->launches += 1;
-        CK(cudaMemcpyAsync(s->h_gst, s->gm_st.p, sizeof(GmresState), cudaMemcpyDeviceToHost, s->stream));
-        CK(cudaStreamSynchronize(s->stream));
+    CHECK_RC(s->gm_vecs.ensure((size_t)stride * nvec));
+    const int one = gmres_one_kernel(s, mk, flex ? augk : -1, stride, rtol, btol, atol, maxit);
+    if (one < 0) return one;
+    if (one > 0) {
         const GmresState &g = *s->h_gst;
-        if (g.status != kStatusDeclined) {
-            s->plan_due = true;
-            if (residual) *residual = g.residual;
-            if (g.status == GMRES_NONFINITE)
-                return fail(PHG_GPU_ERR_NAN, "GMRES: non-finite values after %d iterations", g.nits);
-            if (g.status == kStatusPassLimit)
-                return fail(PHG_GPU_ERR_STATE, "GMRES: the iteration loop exceeded its bound");
-            const int nits = g.nits;
-            CHECK_RC(copy_out(s, x, s->x.p, (size_t)n));
-            CK(cudaStreamSynchronize(s->stream));
-            return nits;
-        }
-        coop_decline(s, COOP_GMRES);
+        if (residual) *residual = g.residual;
+        if (g.status == GMRES_NONFINITE)
+            return fail(PHG_GPU_ERR_NAN, "GMRES: non-finite values after %d iterations", g.nits);
+        if (g.status == kStatusPassLimit)
+            return fail(PHG_GPU_ERR_STATE, "GMRES: the iteration loop exceeded its bound");
+        const int nits = g.nits;
+        CHECK_RC(copy_out(s, x, s->x.p, (size_t)n));
+        CK(cudaStreamSynchronize(s->stream));
+        return nits;
     }
     // ||b|| (solver-phg.c:1071-1075)
     CK(cudaMemsetAsync(s->ticket.p, 0, sizeof(unsigned) * kRedTickets, s->stream));
@@ -2063,7 +2104,6 @@ static int gmres_impl(phgGpuSystem *s, int restart, int augk, double rtol, doubl
         return 0;
     }
     CHECK_RC(tune_spmv(s));
-    CHECK_RC(s->gm_vecs.ensure((size_t)stride * nvec));
     CHECK_RC(s->gm_small.ensure((size_t)gmres_small_doubles(restart)));
     const int R2 = restart + 2;
     GmresState init{};

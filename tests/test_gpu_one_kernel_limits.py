@@ -100,3 +100,80 @@ def test_declined_matrix_is_remembered(gpu, solver):
         assert second == forced > 1
         s.set_matrix(*banded_spd(2000, 3, seed=4))
         assert launches(s, lambda: solve(s, solver))[1] == 1
+
+
+# the launches of the one-kernel solvers, refused as the driver refuses a
+# cooperative grid that cannot be resident (720, too large)
+REFUSE = "".join("int %s(void) { return 720; }\n" % f for f in (
+    "_ZN4phgb15launch_pcg_coopERKNS_6PcgRunEP11CUstream_st",
+    "_ZN4phgb17launch_mixed_coopERKNS_8MixedRunEP11CUstream_st",
+    "_ZN4phgb16launch_bicg_coopERKNS_7BicgRunEP11CUstream_st",
+    "_ZN4phgb17launch_gmres_coopERKNS_8GmresRunEP11CUstream_st",
+    "_ZN4phgb16launch_gear_coopERKNS_11GearBuffersERKNS_7Q16ViewEiPdP11CUstream_st"))
+
+REFUSED_SOLVES = """
+import sys
+sys.path[:0] = sys.argv[1:3]
+import phg_b200
+from oracle import pho
+import test_gpu_one_kernel_limits as t
+A = t.banded_spd(3000, 6, seed=1)
+for solver in t.SOLVERS:
+    with phg_b200.Solver(0) as s:
+        s.set_matrix(*A)
+        for again in range(2):
+            (x, nits), k = t.launches(s, lambda: t.solve(s, solver))
+            assert k > nits, (solver, k)
+            t.check(pho, A, solver, x)
+        if solver == "mixed":   # the cooperative form of the q16 iterations
+            s.set_spmv_plan32("q16", 1)
+            (x, nits), k = t.launches(s, lambda: t.solve(s, solver))
+            assert k > nits, (solver, k)
+            t.check(pho, A, solver, x)
+print("refused and solved")
+"""
+
+
+def test_refused_launch_goes_to_the_launched_path(gpu, tmp_path):
+    """A program whose share of the device cannot hold the grid: every
+    cooperative launch answers "too large" (a preloaded stand-in for the
+    library's launch functions), and every solver still solves."""
+    import os
+    import subprocess
+    import sys
+
+    from conftest import ROOT
+    (tmp_path / "refuse.c").write_text(REFUSE)
+    lib = str(tmp_path / "refuse.so")
+    subprocess.run(["gcc", "-shared", "-fPIC", "-o", lib, str(tmp_path / "refuse.c")], check=True)
+    p = subprocess.run([sys.executable, "-c", REFUSED_SOLVES, ROOT, os.path.join(ROOT, "tests")],
+                       env=dict(os.environ, LD_PRELOAD=lib), capture_output=True, text=True, timeout=300)
+    assert p.returncode == 0 and "refused and solved" in p.stdout, (p.stdout[-2000:], p.stderr[-2000:])
+
+
+def test_no_memory_for_the_matrix_copy(gpu, oracle):
+    """With the product's layout made and less memory free than the kernel's
+    copy of the matrix takes (12 bytes an entry), the launched iteration solves."""
+    import torch
+    A = banded_spd(200000, 30, seed=2)
+    copy = 12 * len(A[1])
+    assert copy > 96 << 20
+    with gpu.Solver(0) as s:
+        s.set_matrix(*A)
+        s.mat_vec(A[3])
+        held, chunk = [], 1 << 34
+        while chunk >= 16 << 20:   # leave 32 to 48 MB
+            free = torch.cuda.mem_get_info()[0]
+            if free - chunk < 32 << 20:
+                chunk >>= 1
+                continue
+            held.append(torch.empty(chunk, dtype=torch.uint8, device="cuda"))
+        try:
+            (x, nits), k = launches(s, lambda: solve(s, "pcg"))
+        finally:
+            del held
+            torch.cuda.empty_cache()
+        assert k > nits
+        check(oracle, A, "pcg", x)
+        # with the memory back, the kernel takes it
+        assert launches(s, lambda: solve(s, "pcg"))[1] == 1
