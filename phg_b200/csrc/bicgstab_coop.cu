@@ -232,14 +232,14 @@ constexpr int64_t kRowBytes = 6 * sizeof(double);   // r / s, rh, p, v, t, diago
 
 }  // namespace
 
-int64_t bicg_coop_entries(int64_t n, int64_t nnz) {
+int64_t bicg_coop_entries(int64_t n, int64_t nnz, int sms) {
     CoopSplit sp;
-    return coop_split(n, nnz, kRowBytes, 0, 4, kSpare, &sp) ? nnz : -1;
+    return coop_split(n, nnz, kRowBytes, 0, 4, kSpare, sms, &sp) ? nnz : -1;
 }
 
 cudaError_t launch_bicg_coop(const BicgRun &R, cudaStream_t s) {
     CoopSplit sp;
-    if (!coop_split(R.A.n, R.nnz, kRowBytes, 0, 4, kSpare, &sp)) return cudaErrorCooperativeLaunchTooLarge;
+    if (!coop_split(R.A.n, R.nnz, kRowBytes, 0, 4, kSpare, R.sms, &sp)) return cudaErrorCooperativeLaunchTooLarge;
     switch (sp.lanes) {
     case 1: return coop_launch(bicg_coop_kernel<1>, R, sp, s);
     case 2: return coop_launch(bicg_coop_kernel<2>, R, sp, s);

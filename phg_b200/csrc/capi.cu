@@ -155,6 +155,7 @@ struct phgGpuSystem_ {
     int device = 0;
     cudaStream_t stream = nullptr;
     bool own_stream = false;
+    int sms = 0;   // multiprocessors the stream's kernels can run on
     // solver graphs without conditional nodes, relaunched by the host per
     // chunk ($PHG_GPU_PLAIN_GRAPHS=1 at creation): profilers do not see the
     // kernels inside conditional nodes
@@ -845,6 +846,7 @@ int phgGpuCreate(int device, void *stream, phgGpuSystem **out) {
         }
     }
     if (rc == PHG_GPU_OK) {
+        s->sms = stream_sms(s->stream);
         cudaError_t e1 = cudaMallocHost((void **)&s->h_st, sizeof(PcgState));
         cudaError_t e2 = cudaMallocHost((void **)&s->h_sums, 4 * sizeof(double));
         cudaError_t e3 = cudaMallocHost((void **)&s->h_status, 3 * sizeof(int));
@@ -945,6 +947,8 @@ int phgGpuSetStream(phgGpuSystem *s, void *stream) {
     } else {
         s->stream = (cudaStream_t)stream;
     }
+    s->sms = stream_sms(s->stream);
+    s->coop_declined = 0;   // the longest row a kernel takes depends on its blocks
     return PHG_GPU_OK;
 }
 
@@ -1381,7 +1385,7 @@ int phgGpuMatVec(phgGpuSystem *s, const double *x, double *y) {
 static int mixed_one_kernel(phgGpuSystem *s, double rtol, double btol, double atol, int maxit) {
     const int64_t n = s->n;
     if (s->plan32_set && s->unroll32 != 0 && s->tuned32_n == n && s->tuned32_nnz == s->nnz) return 0;
-    const int64_t entries = s->coop_declined & COOP_MIXED ? -1 : mixed_coop_entries(n, s->nnz);
+    const int64_t entries = s->coop_declined & COOP_MIXED ? -1 : mixed_coop_entries(n, s->nnz, s->sms);
     if (entries < 0) return 0;
     const int ready = coop_buffers(s, entries, true);
     if (ready <= 0) return ready;
@@ -1389,8 +1393,8 @@ static int mixed_one_kernel(phgGpuSystem *s, double rtol, double btol, double at
     CHECK_RC(s->mixed_out.ensure(1));
     if (s->h_mixed == nullptr) CK(cudaMallocHost((void **)&s->h_mixed, sizeof(MixedResult)));
     const MixedRun run{CsrView{n, s->rp.p, s->ci.p, s->va.p}, s->nnz, s->coop_cols.p, s->coop_vals32.p, s->coop_vals.p,
-                       s->x.p, s->u32.p, s->rhs.p, s->diag.p, rtol, btol, atol, 0.1, maxit, s->coop_xch.p, 0,
-                       s->mixed_out.p};
+                       s->x.p, s->u32.p, s->rhs.p, s->diag.p, rtol, btol, atol, 0.1, maxit, s->coop_xch.p, s->sms,
+                       0, s->mixed_out.p};
     const cudaError_t e = launch_mixed_coop(run, s->stream);
     if (coop_refused(e)) return 0;
     CK(e);
@@ -1732,12 +1736,12 @@ namespace {
 int pcg_one_kernel(phgGpuSystem *s, const double *drhs, double rtol, double btol, double atol, int maxit,
                    double *dhist) {
     const int64_t n = s->n;
-    const int64_t entries = plan_forced(s) || s->coop_declined & COOP_PCG ? -1 : pcg_coop_entries(n, s->nnz);
+    const int64_t entries = plan_forced(s) || s->coop_declined & COOP_PCG ? -1 : pcg_coop_entries(n, s->nnz, s->sms);
     if (entries < 0) return 0;
     const int ready = coop_buffers(s, entries, false);
     if (ready <= 0) return ready;
     const PcgRun run{CsrView{n, s->rp.p, s->ci.p, s->va.p}, s->nnz, s->coop_cols.p, s->coop_vals.p, s->x.p, s->p.p,
-                     s->Ap.p, s->r.p, drhs, s->diag.p, rtol, btol, atol, maxit, dhist, s->coop_xch.p, 0, s->st.p};
+                     s->Ap.p, s->r.p, drhs, s->diag.p, rtol, btol, atol, maxit, dhist, s->coop_xch.p, s->sms, 0, s->st.p};
     const cudaError_t e = launch_pcg_coop(run, s->stream);
     if (coop_refused(e)) return 0;
     CK(e);
@@ -1862,15 +1866,15 @@ int pcg_core(phgGpuSystem *s, const double *drhs, double rtol, double btol, doub
 // or 0 when the kernel does not take it (as pcg_one_kernel).
 int bicg_one_kernel(phgGpuSystem *s, double rtol, double btol, double atol, int maxit, double *dhist) {
     const int64_t n = s->n;
-    const int64_t entries = plan_forced(s) || s->coop_declined & COOP_BICG ? -1 : bicg_coop_entries(n, s->nnz);
+    const int64_t entries = plan_forced(s) || s->coop_declined & COOP_BICG ? -1 : bicg_coop_entries(n, s->nnz, s->sms);
     if (entries < 0) return 0;
     const int ready = coop_buffers(s, entries, false);
     if (ready <= 0) return ready;
     CHECK_RC(s->bicg_st.ensure(1));
     if (s->h_bst == nullptr) CK(cudaMallocHost((void **)&s->h_bst, sizeof(BicgState)));
     const BicgRun run{CsrView{n, s->rp.p, s->ci.p, s->va.p}, s->nnz, s->coop_cols.p, s->coop_vals.p, s->x.p, s->p.p,
-                      s->Ap.p, s->rhs.p, s->diag.p, rtol, btol, atol, maxit, dhist, s->coop_xch.p, 0,
-                      s->bicg_st.p};
+                      s->Ap.p, s->rhs.p, s->diag.p, rtol, btol, atol, maxit, dhist, s->coop_xch.p, s->sms,
+                      0, s->bicg_st.p};
     const cudaError_t e = launch_bicg_coop(run, s->stream);
     if (coop_refused(e)) return 0;
     CK(e);
@@ -2033,7 +2037,7 @@ static int gmres_one_kernel(phgGpuSystem *s, int mk, int augk, int64_t stride, d
     const bool flex = augk >= 0;
     const int restart = flex ? mk + augk : mk;
     const int64_t entries =
-        plan_forced(s) || s->coop_declined & COOP_GMRES ? -1 : gmres_coop_entries(n, s->nnz, restart);
+        plan_forced(s) || s->coop_declined & COOP_GMRES ? -1 : gmres_coop_entries(n, s->nnz, restart, s->sms);
     if (entries < 0) return 0;
     const int ready = coop_buffers(s, entries, false);
     if (ready <= 0) return ready;
@@ -2041,7 +2045,8 @@ static int gmres_one_kernel(phgGpuSystem *s, int mk, int augk, int64_t stride, d
     double *Z1 = flex ? F1 + (int64_t)(restart + 1) * stride : nullptr;
     if (flex) CK(cudaMemsetAsync(Z1, 0, sizeof(double) * (size_t)stride * augk, s->stream));
     const GmresRun run{CsrView{n, s->rp.p, s->ci.p, s->va.p}, s->nnz, s->coop_cols.p, s->coop_vals.p, s->x.p, s->rhs.p,
-                       s->diag.p, V, F1, Z1, stride, rtol, btol, atol, maxit, mk, augk, s->coop_xch.p, 0, s->gm_st.p};
+                       s->diag.p, V, F1, Z1, stride, rtol, btol, atol, maxit, mk, augk, s->coop_xch.p, s->sms, 0,
+                       s->gm_st.p};
     const cudaError_t e = launch_gmres_coop(run, s->stream);
     if (coop_refused(e)) return 0;
     CK(e);

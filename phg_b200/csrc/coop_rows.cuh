@@ -281,7 +281,7 @@ inline int coop_max_row(int64_t nnz, int blocks, int lanes, int spare) {
     return most < kCoopMaxRowLen ? (int)most : kCoopMaxRowLen;
 }
 
-// The launch of a one-kernel solver: blocks, lanes a row, longest row and shared
+// The launch of a one-kernel solver on that many multiprocessors: blocks, lanes a row, longest row and shared
 // memory (`fixed_bytes`, `row_bytes` of vectors a row, and the row bookkeeping);
 // false when it is too large.  `spare`: see coop_max_row, 0 for no limit of the
 // kind.
@@ -301,16 +301,15 @@ struct CoopSplit {
 };
 
 inline bool coop_split(int64_t n, int64_t nnz, int64_t row_bytes, int64_t fixed_bytes, int most_lanes, int spare,
-                       CoopSplit *out) {
-    int dev = 0, coop = 0, sms = 0, most = 0;
+                       int sms, CoopSplit *out) {
+    int dev = 0, coop = 0, most = 0;
     if (cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess) {
         cudaGetLastError();
         return false;
     }
-    if (!coop) return false;
+    if (!coop || sms < 1) return false;
     if (sms > kCoopMaxBlocks) sms = kCoopMaxBlocks;
     const int64_t slices = ceil_div(n, 32);
     int64_t G = ceil_div(nnz + 4 * n, kCoopBlockWork);

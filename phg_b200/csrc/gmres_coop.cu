@@ -264,14 +264,14 @@ constexpr int64_t kRowBytes = 3 * sizeof(double);   // w, z, diagonal
 
 }  // namespace
 
-int64_t gmres_coop_entries(int64_t n, int64_t nnz, int restart) {
+int64_t gmres_coop_entries(int64_t n, int64_t nnz, int restart, int sms) {
     CoopSplit sp;
-    return coop_split(n, nnz, kRowBytes, 8 * dense_doubles(restart), 4, kSpare, &sp) ? nnz : -1;
+    return coop_split(n, nnz, kRowBytes, 8 * dense_doubles(restart), 4, kSpare, sms, &sp) ? nnz : -1;
 }
 
 cudaError_t launch_gmres_coop(const GmresRun &R, cudaStream_t s) {
     CoopSplit sp;
-    if (!coop_split(R.A.n, R.nnz, kRowBytes, 8 * dense_doubles(R.mk + (R.augk >= 0 ? R.augk : 0)), 4, kSpare, &sp))
+    if (!coop_split(R.A.n, R.nnz, kRowBytes, 8 * dense_doubles(R.mk + (R.augk >= 0 ? R.augk : 0)), 4, kSpare, R.sms, &sp))
         return cudaErrorCooperativeLaunchTooLarge;
     switch (sp.lanes) {
     case 1: return coop_launch(gmres_coop_kernel<1>, R, sp, s);

@@ -19,6 +19,7 @@ struct BicgRun {
     int maxit;
     double *hist;        // optional: ||r|| after each iteration
     double *exchange;    // coop_exchange_doubles(), zero before the launch
+    int sms;             // multiprocessors of the stream (stream_sms)
     int max_row;         // a longer row declines the solve; set by the launch
     BicgState *st;       // out: nits, residual, status (BICG_*)
 };
@@ -37,14 +38,15 @@ struct GmresRun {
     double rtol, btol, atol;
     int maxit, mk, augk; // steps of the first cycle, augmenting corrections
     double *exchange;
+    int sms;             // multiprocessors of the stream (stream_sms)
     int max_row;         // a longer row declines the solve; set by the launch
     GmresState *st;      // out: nits, residual, status (GMRES_*, kStatus*)
 };
 
-// Entries of the matrix copy a solve makes on the current device, -1 when it
-// is too large for the kernel.
-int64_t bicg_coop_entries(int64_t n, int64_t nnz);
-int64_t gmres_coop_entries(int64_t n, int64_t nnz, int restart);
+// Entries of the matrix copy a solve makes on sms multiprocessors (stream_sms),
+// -1 when it is too large for the kernel.
+int64_t bicg_coop_entries(int64_t n, int64_t nnz, int sms);
+int64_t gmres_coop_entries(int64_t n, int64_t nnz, int restart, int sms);
 cudaError_t launch_bicg_coop(const BicgRun &R, cudaStream_t s);
 cudaError_t launch_gmres_coop(const GmresRun &R, cudaStream_t s);
 

@@ -31,6 +31,7 @@
 #include "common.cuh"
 #include "grid_sync.cuh"
 #include "mixed.h"
+#include "pcg_coop.h"
 #include "reduce.cuh"
 #include "rows.cuh"
 
@@ -431,10 +432,10 @@ gear_coop_kernel(const Q16View Q, const GearBuffers B, double *exchange) {
 
 cudaError_t launch_gear_coop(const GearBuffers &B, const Q16View &Q, int unroll, double *exchange, cudaStream_t s) {
     auto kernel = unroll == 2 ? gear_coop_kernel<2> : gear_coop_kernel<1>;
-    int dev = 0, coop = 0, sms = 0, per_sm = 0;
+    int dev = 0, coop = 0, per_sm = 0;
+    const int sms = stream_sms(s);
     cudaError_t e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
-    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kGearCoopThreads, 0);
     if (e != cudaSuccess) return e;
     int grid = sms * per_sm < kCoopMostBlocks ? sms * per_sm : kCoopMostBlocks;

@@ -235,14 +235,14 @@ constexpr int64_t kMaxEntries = 10000000;
 
 }  // namespace
 
-int64_t mixed_coop_entries(int64_t n, int64_t nnz) {
+int64_t mixed_coop_entries(int64_t n, int64_t nnz, int sms) {
     CoopSplit sp;
-    return nnz <= kMaxEntries && coop_split(n, nnz, kRowBytes, 0, 2, 0, &sp) ? nnz : -1;
+    return nnz <= kMaxEntries && coop_split(n, nnz, kRowBytes, 0, 2, 0, sms, &sp) ? nnz : -1;
 }
 
 cudaError_t launch_mixed_coop(const MixedRun &R, cudaStream_t s) {
     CoopSplit sp;
-    if (!coop_split(R.A.n, R.nnz, kRowBytes, 0, 2, 0, &sp)) return cudaErrorCooperativeLaunchTooLarge;
+    if (!coop_split(R.A.n, R.nnz, kRowBytes, 0, 2, 0, R.sms, &sp)) return cudaErrorCooperativeLaunchTooLarge;
     return sp.lanes == 1 ? coop_launch(mixed_coop_kernel<1>, R, sp, s) : coop_launch(mixed_coop_kernel<2>, R, sp, s);
 }
 

@@ -23,13 +23,14 @@ struct MixedRun {
     double rtol, btol, atol, delta;
     int maxit;
     double *exchange;    // coop_exchange_doubles(), zero before the launch
+    int sms;             // multiprocessors of the stream (stream_sms)
     int max_row;         // a longer row declines the solve; set by the launch
     MixedResult *out;
 };
 
-// Entries of the matrix copy a solve of n rows and nnz entries makes on the
-// current device, -1 when it is too large for the kernel.
-int64_t mixed_coop_entries(int64_t n, int64_t nnz);
+// Entries of the matrix copy a solve of n rows and nnz entries makes on sms
+// multiprocessors (stream_sms), -1 when it is too large for the kernel.
+int64_t mixed_coop_entries(int64_t n, int64_t nnz, int sms);
 cudaError_t launch_mixed_coop(const MixedRun &R, cudaStream_t s);
 
 }  // namespace phgb

@@ -28,6 +28,7 @@
 #include "grid_sync.cuh"
 #include "pcg_coop.h"
 
+#include <cudaTypedefs.h>
 #include <float.h>
 #include <math.h>
 
@@ -225,14 +226,48 @@ constexpr int64_t kFusedEntries = 1500000;
 
 int coop_exchange_doubles() { return kCoopDoubles; }
 
-int64_t pcg_coop_entries(int64_t n, int64_t nnz) {
+int stream_sms(cudaStream_t s) {
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    struct Driver {
+        PFN_cuStreamGetGreenCtx_v12040 context = nullptr;
+        PFN_cuGreenCtxGetDevResource_v12040 resource = nullptr;
+        static void *entry(const char *name) {
+            void *f = nullptr;
+            cudaDriverEntryPointQueryResult found;
+            if (cudaGetDriverEntryPointByVersion(name, &f, 12040, cudaEnableDefault, &found) != cudaSuccess) {
+                cudaGetLastError();
+                return nullptr;
+            }
+            return found == cudaDriverEntryPointSuccess ? f : nullptr;
+        }
+        Driver() {
+            context = (PFN_cuStreamGetGreenCtx_v12040)entry("cuStreamGetGreenCtx");
+            resource = (PFN_cuGreenCtxGetDevResource_v12040)entry("cuGreenCtxGetDevResource");
+        }
+    };
+    static const Driver driver;
+    CUgreenCtx green = nullptr;
+    CUdevResource r{};
+    if (driver.context != nullptr && driver.resource != nullptr &&
+        driver.context((CUstream)s, &green) == CUDA_SUCCESS && green != nullptr &&
+        driver.resource(green, &r, CU_DEV_RESOURCE_TYPE_SM) == CUDA_SUCCESS && (int)r.sm.smCount < sms)
+        sms = (int)r.sm.smCount;
+    return sms;
+}
+
+int64_t pcg_coop_entries(int64_t n, int64_t nnz, int sms) {
     CoopSplit sp;
-    return coop_split(n, nnz, kRowBytes, 0, 4, kSpare, &sp) ? nnz : -1;
+    return coop_split(n, nnz, kRowBytes, 0, 4, kSpare, sms, &sp) ? nnz : -1;
 }
 
 cudaError_t launch_pcg_coop(const PcgRun &R, cudaStream_t s) {
     CoopSplit sp;
-    if (!coop_split(R.A.n, R.nnz, kRowBytes, 0, 4, kSpare, &sp)) return cudaErrorCooperativeLaunchTooLarge;
+    if (!coop_split(R.A.n, R.nnz, kRowBytes, 0, 4, kSpare, R.sms, &sp)) return cudaErrorCooperativeLaunchTooLarge;
     if (R.nnz <= kFusedEntries) {
         switch (sp.lanes) {
         case 1: return coop_launch(pcg_coop_kernel<1, true>, R, sp, s);

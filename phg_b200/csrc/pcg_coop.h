@@ -17,15 +17,21 @@ struct PcgRun {
     int maxit;
     double *hist;        // optional: ||r|| after each iteration, [0] = ||r0||
     double *exchange;    // coop_exchange_doubles(), zero before the launch
+    int sms;             // multiprocessors of the stream (stream_sms)
     int max_row;         // a longer row declines the solve; set by the launch
     PcgState *st;        // out: nits, residual, status
 };
 
 int coop_exchange_doubles();
 
-// Entries of the matrix copy a solve of n rows and nnz entries makes on the
-// current device, -1 when it is too large for the kernel.
-int64_t pcg_coop_entries(int64_t n, int64_t nnz);
+// Multiprocessors that kernels of the stream can run on: the device's, or those
+// of the green context the stream belongs to (pcg_coop.cu).  A grid of more
+// blocks than these hold would wait for blocks that are not resident.
+int stream_sms(cudaStream_t s);
+
+// Entries of the matrix copy a solve of n rows and nnz entries makes on sms
+// multiprocessors (stream_sms), -1 when it is too large for the kernel.
+int64_t pcg_coop_entries(int64_t n, int64_t nnz, int sms);
 cudaError_t launch_pcg_coop(const PcgRun &R, cudaStream_t s);
 
 }  // namespace phgb

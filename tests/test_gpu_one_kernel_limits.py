@@ -177,3 +177,36 @@ def test_no_memory_for_the_matrix_copy(gpu, oracle):
         check(oracle, A, "pcg", x)
         # with the memory back, the kernel takes it
         assert launches(s, lambda: solve(s, "pcg"))[1] == 1
+
+
+def test_stream_with_part_of_the_device(gpu, oracle):
+    """A system on a stream that has 16 multiprocessors (a green context): the
+    grids fit them, so the solves run as one kernel there too, the cooperative
+    form of the q16 iterations among them."""
+    import torch
+    drv = pytest.importorskip("cuda.bindings.driver")
+
+    def call(result):
+        assert result[0] == drv.CUresult.CUDA_SUCCESS, result[0]
+        return result[1] if len(result) == 2 else result[1:]
+
+    torch.cuda.init()
+    torch.zeros(1, device="cuda")
+    dev = call(drv.cuDeviceGet(0))
+    sms = call(drv.cuDeviceGetDevResource(dev, drv.CUdevResourceType.CU_DEV_RESOURCE_TYPE_SM))
+    groups = call(drv.cuDevSmResourceSplitByCount(1, sms, 0, 16))[0]
+    desc = call(drv.cuDevResourceGenerateDesc([groups[0]], 1))
+    green = call(drv.cuGreenCtxCreate(desc, dev, int(drv.CUgreenCtxCreate_flags.CU_GREEN_CTX_DEFAULT_STREAM)))
+    stream = call(drv.cuGreenCtxStreamCreate(green, int(drv.CUstream_flags.CU_STREAM_NON_BLOCKING), 0))
+    A = banded_spd(40001, 12, seed=7)
+    for solver in SOLVERS:
+        with gpu.Solver(0, stream=int(stream)) as s:
+            s.set_matrix(*A)
+            (x, _), k = launches(s, lambda: solve(s, solver))
+            assert k == 1, solver
+            check(oracle, A, solver, x)
+            if solver == "mixed":
+                s.set_spmv_plan32("q16", 1)
+                check(oracle, A, solver, solve(s, solver)[0])
+    drv.cuStreamDestroy(stream)
+    drv.cuGreenCtxDestroy(green)
