@@ -1385,7 +1385,8 @@ int phgGpuMatVec(phgGpuSystem *s, const double *x, double *y) {
 static int mixed_one_kernel(phgGpuSystem *s, double rtol, double btol, double atol, int maxit) {
     const int64_t n = s->n;
     if (s->plan32_set && s->unroll32 != 0 && s->tuned32_n == n && s->tuned32_nnz == s->nnz) return 0;
-    const int64_t entries = s->coop_declined & COOP_MIXED ? -1 : mixed_coop_entries(n, s->nnz, s->sms);
+    const int64_t entries =
+        plan_forced(s) || s->coop_declined & COOP_MIXED ? -1 : mixed_coop_entries(n, s->nnz, s->sms);
     if (entries < 0) return 0;
     const int ready = coop_buffers(s, entries, true);
     if (ready <= 0) return ready;

@@ -210,3 +210,18 @@ def test_stream_with_part_of_the_device(gpu, oracle):
                 check(oracle, A, solver, solve(s, solver)[0])
     drv.cuStreamDestroy(stream)
     drv.cuGreenCtxDestroy(green)
+
+
+def test_mixed_solve_on_an_fp64_layout_of_the_caller(gpu, oracle):
+    """phgGpuSetSpMVPlan holds for the mixed solve too, whose FP64 residuals
+    take that layout: it goes to the launched iteration."""
+    A = banded_spd(3000, 6, seed=8)
+    with gpu.Solver(0) as s:
+        s.set_matrix(*A)
+        assert launches(s, lambda: solve(s, "mixed"))[1] == 1
+        for layout, param in (("csr", 8), ("sell", 4), ("q16", 1)):
+            s.set_spmv_plan(layout, param)
+            (x, _), k = launches(s, lambda: solve(s, "mixed"))
+            assert k > 5, layout
+            check(oracle, A, "mixed", x)
+            assert s.spmv_plan()[:2] == (layout, param)
