@@ -284,10 +284,13 @@ struct phgGpuSystem_ {
     DevBuf<float> bY32, bR32, bP32, bAP32, bva32;
     DevBuf<int> bint;
     DevBuf<unsigned> btick;
-    int btile = 0;                      // autotuned SpMM tile (columns)
-    int64_t btile_n = -1, btile_nnz = -1;
-    int btile_K = -1;
-    double btile_ms[4] = {};
+    struct BlockTile {
+        int tile = 0;                   // autotuned SpMM tile (columns)
+        int64_t n = -1, nnz = -1;
+        int K = -1;
+        double ms[4] = {};
+    } btile[2];                         // of the FP64 and the FP32 product
+    int btile_last = 0;                 // the last solve's
     cudaGraphExec_t graph_block = nullptr;
     GraphKey gkey_block{};
     DevBuf<float> u32, s32;             // mixed solver: u = D^-1 r, s = A p
@@ -2299,8 +2302,10 @@ int phgGpuSolverBlockPCG(phgGpuSystem *s, int nrhs, const double *B, double *X, 
     V.va32 = s->bva32.p; V.D32 = s->D32.p; V.Y32 = s->bY32.p; V.R32 = s->bR32.p; V.P32 = s->bP32.p;
     V.AP32 = s->bAP32.p;
 
-    // autotune the SpMM tile once per matrix shape and column count
-    if (!(s->btile != 0 && s->btile_n == n && s->btile_nnz == s->nnz && s->btile_K == K)) {
+    // autotune the SpMM tile once per matrix shape, column count and precision
+    s->btile_last = mixed ? 1 : 0;
+    auto &bt = s->btile[s->btile_last];
+    if (!(bt.tile != 0 && bt.n == n && bt.nnz == s->nnz && bt.K == K)) {
         CK(cudaMemsetAsync(s->bP.p, 0, sizeof(double) * nk, s->stream));
         CK(cudaMemsetAsync(s->bint.p, 0, sizeof(int) * (3 * 64 + 8), s->stream));   // flags: not done
         cudaEvent_t a, b;
@@ -2309,7 +2314,7 @@ int phgGpuSolverBlockPCG(phgGpuSystem *s, int nrhs, const double *B, double *X, 
         const int cand[4] = {8, 16, 32, 64};
         int best = -1;
         for (int c = 0; c < 4; c++) {
-            s->btile_ms[c] = 0.0;
+            bt.ms[c] = 0.0;
             if (cand[c] > K) continue;
             for (int i = 0; i < 2; i++) {
                 if (mixed) CK(launch_block_spmm32(P, cand[c], s->bva32.p, s->bP32.p, s->bAP32.p, s->stream));
@@ -2324,16 +2329,16 @@ int phgGpuSolverBlockPCG(phgGpuSystem *s, int nrhs, const double *B, double *X, 
             CK(cudaEventSynchronize(b));
             float ms = 0;
             CK(cudaEventElapsedTime(&ms, a, b));
-            s->btile_ms[c] = ms / 3;
+            bt.ms[c] = ms / 3;
             s->launches += 5;
-            if (best < 0 || s->btile_ms[c] < s->btile_ms[best]) best = c;
+            if (best < 0 || bt.ms[c] < bt.ms[best]) best = c;
         }
         cudaEventDestroy(a);
         cudaEventDestroy(b);
-        s->btile = cand[best < 0 ? 0 : best];
-        s->btile_n = n; s->btile_nnz = s->nnz; s->btile_K = K;
+        bt.tile = cand[best < 0 ? 0 : best];
+        bt.n = n; bt.nnz = s->nnz; bt.K = K;
     }
-    const int T = s->btile;
+    const int T = bt.tile;
 
     // R = B (zero initial guess), X = 0
     const double *dB;
@@ -2400,10 +2405,11 @@ int phgGpuSolverBlockPCG(phgGpuSystem *s, int nrhs, const double *B, double *X, 
 
 int phgGpuGetBlockTile(phgGpuSystem *s, int *tile, double *times_ms) {
     if (s == nullptr) return fail(PHG_GPU_ERR_ARG, "null system");
-    if (s->btile == 0) return fail(PHG_GPU_ERR_STATE, "no block solve yet");
-    if (tile) *tile = s->btile;
+    const auto &bt = s->btile[s->btile_last];
+    if (bt.tile == 0) return fail(PHG_GPU_ERR_STATE, "no block solve yet");
+    if (tile) *tile = bt.tile;
     if (times_ms)
-        for (int c = 0; c < 4; c++) times_ms[c] = s->btile_ms[c];
+        for (int c = 0; c < 4; c++) times_ms[c] = bt.ms[c];
     return PHG_GPU_OK;
 }
 }  // extern "C"

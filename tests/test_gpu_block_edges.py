@@ -30,3 +30,22 @@ def test_block_edges(gpu, oracle, n, nrhs, mixed):
         assert np.linalg.norm(X[:, k] - xo) <= 1e3 * rtol * np.linalg.norm(xo)
         r = np.linalg.norm(bk - oracle.spmv(ptr, cols, vals, np.ascontiguousarray(X[:, k])))
         assert abs(res[k] - r) <= 1e-13 * np.linalg.norm(bk)
+
+
+def test_tile_of_each_precision(gpu):
+    """The FP64 and the FP32 product have tiles of their own: the first solve
+    in either precision times the four tiles of 64 columns (five launches
+    each), whichever came first, and later ones keep both choices."""
+    ptr, cols, vals, b = banded_spd(1000, 6, seed=9)
+    B = np.random.default_rng(1).standard_normal((1000, 64))
+    with gpu.Solver(0) as s:
+        s.set_matrix(ptr, cols, vals, b)
+
+        def count(mixed):
+            before = s.launch_count()
+            s.solve_block_pcg(B, rtol=1e-8, mixed=mixed)
+            return s.launch_count() - before, s.block_tile()
+        k32, t32 = count(True)
+        k64, t64 = count(False)
+        assert count(True) == (k32 - 20, t32)
+        assert count(False) == (k64 - 20, t64)
