@@ -70,11 +70,15 @@ void warn(const char *fmt, ...) {
             return rc_;           \
     } while (0)
 
-// A device buffer that only grows.
+// A device buffer that only grows, freed with its owner.
 template <typename T>
 struct DevBuf {
     T *p = nullptr;
     size_t cap = 0;
+    DevBuf() = default;
+    DevBuf(const DevBuf &) = delete;
+    DevBuf &operator=(const DevBuf &) = delete;
+    ~DevBuf() { release(); }
     int ensure(size_t n) {
         if (n <= cap && p != nullptr) return PHG_GPU_OK;
         if (p != nullptr) cudaFree(p);
@@ -881,57 +885,14 @@ int phgGpuDestroy(phgGpuSystem *s) {
     if (s->h_bst) cudaFreeHost(s->h_bst);
     if (s->graph_gmres != nullptr) cudaGraphExecDestroy(s->graph_gmres);
     if (s->h_gst) cudaFreeHost(s->h_gst);
-    s->gm_vecs.release();
-    s->gm_small.release();
-    s->gm_st.release();
-    s->bicg_vecs.release();
-    s->bicg_st.release();
-    DevBuf<float> *fbufs[] = {&s->r32, &s->p32, &s->Ap32, &s->y32, &s->D32, &s->sell_vals32, &s->sell2_vals};
-    s->sell2_ssz.release(); s->sell2_sptr.release(); s->sell2_cols.release();
-    s->sell2_order.release(); s->sell2_perm.release(); s->sell2_width.release(); s->sell2_len.release();
-    for (auto *b : fbufs) b->release();
-    s->sell_perm.release(); s->sell_ssz.release(); s->sell_sptr.release(); s->sell_cols.release();
-    s->sell_len.release(); s->sell_vals.release(); s->gst.release(); s->u32.release(); s->s32.release();
-    DevBuf<int32_t> *qi[] = {&s->q16_ssz, &s->q16_sptr, &s->q16_perm, &s->q16_b0, &s->q16_b1};
-    for (auto *b : qi) b->release();
-    DevBuf<uint16_t> *qu[] = {&s->q16_len, &s->q16_split, &s->q16_cols};
-    for (auto *b : qu) b->release();
-    s->q16_v32.release(); s->q16_v64.release(); s->q16_nofit.release();
     if (s->h_nofit) cudaFreeHost(s->h_nofit);
-    s->adj_u.release(); s->adj_uobs.release(); s->adj_rhs.release(); s->adj_lambda.release(); s->adj_grad.release();
     if (s->graph_block != nullptr) cudaGraphExecDestroy(s->graph_block);
-    DevBuf<double> *bb[] = {&s->bX, &s->bR, &s->bP, &s->bAP, &s->bB, &s->bscal, &s->bpart};
-    for (auto *b : bb) b->release();
-    DevBuf<float> *bf[] = {&s->bY32, &s->bR32, &s->bP32, &s->bAP32, &s->bva32};
-    for (auto *b : bf) b->release();
-    s->bint.release();
-    s->btick.release();
-    DevBuf<double> *dbufs[] = {&s->verts, &s->gk, &s->brt, &s->bw, &s->mt, &s->Ke, &s->Re, &s->kappa, &s->f,
-                               &s->g, &s->geo, &s->va, &s->bva, &s->rhs, &s->diag, &s->x, &s->r, &s->p, &s->Ap,
-                               &s->partials, &s->hist, &s->sums};
-    for (auto *b : dbufs) b->release();
-    DevBuf<int32_t> *ibufs[] = {&s->elems, &s->e2l, &s->inc_ptr, &s->inc, &s->cnt, &s->cursor, &s->cnt_keep,
-                                &s->cnt_bdry, &s->rp, &s->ci, &s->brp, &s->bci};
-    for (auto *b : ibufs) b->release();
-    s->bdry.release();
-    s->sc_cols.release();
-    s->sc_vals.release();
-    s->scan_ws.release();
-    s->tmp64.release();
-    s->st.release();
-    s->ticket.release();
-    s->coop_xch.release();
-    s->coop_cols.release();
-    s->coop_vals.release();
-    s->coop_vals32.release();
-    s->mixed_out.release();
     if (s->h_mixed) cudaFreeHost(s->h_mixed);
-    s->status.release();
     if (s->h_st) cudaFreeHost(s->h_st);
     if (s->h_sums) cudaFreeHost(s->h_sums);
     if (s->h_status) cudaFreeHost(s->h_status);
     if (s->own_stream && s->stream != nullptr) cudaStreamDestroy(s->stream);
-    delete s;
+    delete s;   // and its device buffers
     return PHG_GPU_OK;
 }
 
