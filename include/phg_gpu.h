@@ -271,6 +271,18 @@ int phgGpuSolverPCGMixed(phgGpuSystem *sys, double rtol, double btol,
 			 double atol, int maxit, double *x, double *residual,
 			 int *nupdates);
 
+/* How the solvers run.  A system whose vectors fit the shared memory of the
+ * stream's multiprocessors (on a B200 PCG up to 601,000 rows, BiCGstab 407,000,
+ * GMRES some 770,000, mixed PCG 680,000 and 10 million entries) is solved by one
+ * cooperative kernel, and so is a larger mixed solve on the 16-bit-column layout.
+ * The kernel holds its multiprocessors until the solve ends: work on other
+ * streams of the device may have to wait for it.  A program that needs such work
+ * to proceed during a solve sets the product layout (phgGpuSetSpMVPlan; for the
+ * mixed solver phgGpuSetSpMVPlan32 with SELL or pair): solves on a layout of the
+ * caller are launched iteration by iteration, as are those of larger systems, of
+ * matrices with a few rows far longer than the others (PCG, BiCGstab, GMRES), and
+ * where the device cannot hold the kernel's blocks or its copy of the matrix. */
+
 /* The SpMV layout the autotuner chose for the current matrix (no
  * counterpart in the reference): at the first product or launched solve for a
  * matrix shape (a solve that runs as one kernel needs no layout; after one, this

@@ -287,12 +287,21 @@ inline int coop_max_row(int64_t nnz, int blocks, int lanes, int spare) {
 // kind.
 //
 // Shared memory a solve takes at most: what it takes the L1 cache loses, and
-// the product's gathers need that.  With 122 KB a block (P2, 531k rows) an
-// iteration of the FP64 PCG takes 38.5 us (58.5 as separate launches); with 208
-// KB, in an earlier form of the product, 71 against 47.5.
+// the product's gathers need that.  A careful line, the kernels are faster some
+// way beyond it: FP64 PCG, us per iteration in one kernel / launched, 121 KB a
+// block (P2 531k rows) 38.5 / 58.0, 125 KB (P3 551k) 59.0 / 91.5, and with the
+// limit raised 154 KB (P3 681k) 74.6 / 107, 159 KB (P1 705k) 28.2 / 44.4, (P2 705k)
+// 51.0 / 72.7, 188 KB (P3 831k) 105 / 125, 194 KB (P2 857k) 69.7 / 72.2, 206 KB (P1
+// 913k) 51.0 / 48.2; BiCGstab 130 KB (P3 389k) 96.7 / 169, 183 KB (P3 551k) 154 / 220.
 constexpr int64_t kCoopMaxSmem = 136 * 1024;
 // A block per this many entries (a row's vector work counted as four) while
-// there are SMs: below that the barriers of more blocks cost what they save.
+// there are SMs.  Us per iteration with 1024 / 2048 / 4096 / 8192: FP64 PCG P1 343
+// rows 6.6 / 6.5 / 3.3 / 3.4 (one block, no barriers, from 4096 on), P1 729 6.6 /
+// 6.6 / 6.8 / 4.6, P1 3.4k 6.3 / 6.4 / 6.6 / 7.8, P1 36k 6.7 / 6.7 / 6.7 / 8.3, P2
+// 6.9k 8.1 / 8.0 / 8.4 / 9.5, P3 15.6k 12.7 / 12.8 / 12.3 / 13.2; mixed P1 9.3k 6.7 /
+// 6.7 / 7.3 / 7.7; GMRES P1 343 18.4 / 18.2 / 8.1 / 8.0, P1 3.4k 20.3 / 20.3 / 20.5 /
+// 21.8: more blocks than 4096 gives save next to nothing, and cost the smallest
+// systems their barriers.
 constexpr int64_t kCoopBlockWork = 4096;
 
 struct CoopSplit {

@@ -16,6 +16,15 @@
 // polling 148 words each cost 5 us an iteration, after the count nothing.)
 // sync(): the barrier alone, before a vector that other blocks read.
 //
+// While such a grid runs it holds the SMs it has blocks on: 1024 threads of up
+// to 64 registers are an SM's whole register file, so a solve that has a block on
+// every SM (from 606,000 entries on, a row counted as four) lets nothing of
+// another stream run until it ends.  A small kernel of another stream waits up to
+// the whole solve (2000 iterations of P2 250k rows: 42 ms, 0.05 ms beside the
+// launched ones).  Two threads solving at once: P2 250k rows, 100 iterations each,
+// 4.65 ms a pair (6.58 as launches), P1 36k 1.40 (2.24), P1 9k, whose grids fit
+// side by side, 0.74 (1.95).
+//
 // The kernels are launched cooperatively (all blocks resident), so a poll
 // ends; a bound on the polls turns a fault elsewhere into an error status
 // instead of a hang.

@@ -290,7 +290,8 @@ gear_update_kernel(const GearBuffers B, cudaGraphConditionalHandle hif) {
 // the update's bytes: launches, ramps, two ticket sums and a conditional node.
 // Per iteration, us: P2 64^3 (2.1 million rows, 57 million entries) 104 (107 as
 // launches), P2 705k rows 48.9 (51.3), P1 1.03 million rows 35.8 (41.1); the
-// product's blocks finish some 10 us apart at 64^3.  (One block an SM with 64
+// product's blocks finish some 10 us apart at 64^3, and at 32 registers the kernel
+// spills 388 bytes, most of it the partials its sums add.  (One block an SM with 64
 // registers and twice the unrolling: 145 us at P2 64^3.)
 constexpr int kGearCoopThreads = 1024;
 

@@ -229,8 +229,11 @@ mixed_coop_kernel(const MixedRun R) {
 
 constexpr int64_t kRowBytes = 7 * sizeof(float);   // r, u, w, p, s, y, diagonal
 // Entries up to which the FP32 copy (8 bytes each) stays in L2 beside the
-// vectors; beyond, the launched products on the 16-bit-column layout move a
-// quarter fewer bytes from memory.
+// vectors; beyond, the products on the 16-bit-column layout move a quarter fewer
+// bytes from memory.  A careful line, the kernel is faster beyond it too where
+// its vectors fit: us per iteration in one kernel / on the layouts, P2 9.9 million
+// entries 26.4 / 47.4, and with the limit raised P1 10.4 million 26.6 / 30.9, P2
+// 13.7 million 33.3 / 41.6, P3 10.9 million 29.5 / 67.3, 16.5 million 39.9 / 79.3.
 constexpr int64_t kMaxEntries = 10000000;
 
 }  // namespace

@@ -12,15 +12,18 @@
 // Where a barrier costs more than gathers (FUSED, small systems), z goes through
 // L2 too and the product gathers z + beta p from z and the last direction, so
 // that the direction needs no barrier of its own; the values are the same.
-// What bounds it: at 1,000 to 40,000 rows the three barriers, about 1.4 us each,
-// and the latency of the phases between them; from 100,000 rows on the product,
-// which reads the matrix from L2 (up to some 10 million entries) at the rate
-// its gathers allow.  Time per iteration against the same recurrence as three
-// launches in a graph loop: P1 1,331 rows 6.7 us (16.3), P1 36k 6.9 (18.9), P1
-// 133k 10.4 (20.7), P1 389k 18.5 (33.3), P2 69k 11.3 (23.4), P2 250k 22.5
-// (37.4), P2 531k 38.5 (58.5), P3 227k 30.8 (52.2); and a solve needs no tuned
-// layout, no graph and one host wait: 71 us instead of 180 before the first
-// iteration.  (Measured and left: the rows in one contiguous run per block, as
+// What bounds it: up to 40,000 rows the barriers, about 1.4 us each (two in the
+// FUSED form, which systems of that size take up to 1.5 million entries, three
+// otherwise), and the latency of the phases between them: at P1 36k rows a warp
+// waits at a barrier 27 of the 38 cycles it spends on an instruction.  From
+// 100,000 rows on the product, which reads the matrix from L2 (up to some 10
+// million entries) at the rate its gathers allow: at P2 531k rows 42% of the DRAM
+// rate, 55% of L1's, 10 of 21 cycles waiting for loads and 4 at barriers.  Time
+// per iteration against the same recurrence as three launches in a graph loop: P1
+// 1,331 rows 6.7 us (16.3), P1 36k 6.9 (18.9), P1 133k 10.4 (20.7), P1 389k 18.5
+// (33.3), P2 69k 11.3 (23.4), P2 250k 22.5 (37.4), P2 531k 38.5 (58.5), P3 227k
+// 30.8 (52.2); and a solve needs no tuned layout, no graph and one host wait: 71
+// us instead of 180 before the first iteration.  (Measured and left: the rows in one contiguous run per block, as
 // CSR rows of 4 to 16 lanes, as a stream over the entries, or sorted by length:
 // 25 to 29 us on P1 389k and over 100 on P2 531k, whose vertex rows then sit on
 // a third of the blocks.)
@@ -215,6 +218,7 @@ pcg_coop_kernel(const PcgRun R) {
 }
 
 constexpr int kSpare = 72;   // coop_max_row
+// Shared memory takes 601,472 rows on 148 SMs (127 slices of 1,092 bytes a block).
 constexpr int64_t kRowBytes = 4 * sizeof(double);   // r, w / z, p, diagonal
 // Entries up to which the product forms the direction from the two vectors it
 // gathers, saving a barrier: us per iteration with / without, P1 9k rows 6.8 /
