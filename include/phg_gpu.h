@@ -275,8 +275,9 @@ int phgGpuSolverPCGMixed(phgGpuSystem *sys, double rtol, double btol,
  * stream's multiprocessors (on a B200 PCG up to 601,000 rows, BiCGstab 407,000,
  * GMRES some 770,000, mixed PCG 680,000 and 10 million entries) is solved by one
  * cooperative kernel, and so is a larger mixed solve on the 16-bit-column layout.
- * The kernel holds its multiprocessors until the solve ends: work on other
- * streams of the device may have to wait for it.  A program that needs such work
+ * The kernel starts when its multiprocessors are free and holds them until the
+ * solve ends: work on other streams of the device may have to wait for it, and it
+ * waits for theirs.  A program that needs such work
  * to proceed during a solve sets the product layout (phgGpuSetSpMVPlan; for the
  * mixed solver phgGpuSetSpMVPlan32 with SELL or pair): solves on a layout of the
  * caller are launched iteration by iteration, as are those of larger systems, of
